@@ -25,13 +25,13 @@ DEFAULT_REFERENCE = "/root/reference"
 
 def reference_root():
     """The reference checkout ($UMAG_REFERENCE, else the default location), or
-    None when neither exists (the GPU box has no reference tree)."""
+    None when neither holds its kernels (the GPU box has no reference tree)."""
     env = os.environ.get("UMAG_REFERENCE")
     if env:
         if not os.path.isdir(env):
             raise FileNotFoundError(f"UMAG_REFERENCE={env} is not a directory")
         return env
-    return DEFAULT_REFERENCE if os.path.isdir(DEFAULT_REFERENCE) else None
+    return DEFAULT_REFERENCE if os.path.isdir(os.path.join(DEFAULT_REFERENCE, "kernels_src")) else None
 
 
 def _kernels_src():
