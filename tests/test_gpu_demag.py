@@ -156,3 +156,73 @@ def test_pbc_film_of_uniform_m_is_thin_film_limit(cl):
     bz = float(B[2].mean()) / (G.MU0 * 8e5)
     assert abs(bz + 1.0) < 0.02, bz
     d.Free()
+
+
+# line lengths: shortest, longest of each number of stages, one cell below,
+# at and above a length (the next longer one, zero cells read as padding)
+LINE_SIZES = [(1, 1, 1), (4, 3, 2), (7, 8, 5), (8, 7, 6), (9, 9, 7), (15, 16, 8), (16, 15, 9), (18, 18, 10),
+              (48, 24, 11), (50, 49, 12), (52, 50, 1), (63, 64, 16), (64, 65, 14), (96, 60, 1), (99, 100, 3),
+              (110, 98, 1), (128, 120, 1), (130, 126, 1), (200, 192, 1), (192, 200, 1), (210, 220, 1), (240, 250, 1),
+              (320, 256, 1), (36, 300, 1), (390, 40, 1), (24, 512, 1), (640, 12, 1), (10, 650, 1), (8, 1024, 1),
+              (1024, 6, 1), (13, 11, 32), (64, 16, 20), (5, 4, 24)]
+
+
+@pytest.mark.parametrize("N", LINE_SIZES)
+def test_line_transforms_match_oracle(cl, N):
+    """Every stage count and remainder of the line transforms against the
+    oracle's FP64 field.  The float32 transforms are about 1e-7 of max|B| off
+    (three axes of log2 N rounded butterflies); an index or twiddle mistake
+    is of order 1."""
+    assert _check_field(cl, N, (2e-9, 3e-9, 2.5e-9), 8e5) <= 2e-6
+
+
+def test_odd_rows_with_maps_and_unaligned_field(cl):
+    """Odd Nx (rows not on 8 bytes), per-cell Ms and geometry, and arrays that start 4 bytes off."""
+    N, cell = (27, 10, 3), (2e-9, 2e-9, 2e-9)
+    rng = np.random.default_rng(4)
+    Ms, vol = 6e5 + 3e5 * rng.random(N[::-1]), rng.random(N[::-1])
+    assert _check_field(cl, N, cell, Ms, vol) <= TOL_FIELD
+    N = (32, 10, 3)
+    n = N[0] * N[1] * N[2]
+    d = cl.NewNewellDemag(N, (0, 0, 0), cell)
+    m = cu(G.random_unit(N, 5))
+    want, got = torch.empty_like(m), torch.zeros(3 * n + 1, device="cuda")
+    d.Exec(want, m, None, 8e5)
+    off = torch.zeros(3 * n + 1, device="cuda")
+    off[1:] = m.reshape(-1)
+    d.Exec(got[1:].reshape(m.shape), off[1:].reshape(m.shape), None, 8e5)
+    assert torch.equal(got[1:].reshape(m.shape), want)  # the same arithmetic, other load widths
+    d.Free()
+
+
+@pytest.mark.parametrize("N", [(9, 7, 4), (16, 18, 7), (64, 64, 1)])
+def test_callers_kernel_gives_the_same_plan(cl, N):
+    """A plan from the Newell tensor handed over on the reference's padded grid (which the
+    passes may lengthen) gives the Newell plan's field and the same spectrum back."""
+    cell = (2e-9, 2e-9, 3e-9)
+    d = cl.NewNewellDemag(N, (0, 0, 0), cell)
+    e = cl.NewDemag(N, d.kernel())
+    assert d.padded_size() == e.padded_size() == O.pad_size(N)
+    assert np.array_equal(d.spectrum(), e.spectrum())
+    m = cu(G.random_unit(N, 6))
+    a, b = torch.empty_like(m), torch.empty_like(m)
+    d.Exec(a, m, None, 8e5)
+    e.Exec(b, m, None, 8e5)
+    assert torch.equal(a, b)
+    d.Free()
+    e.Free()
+
+
+@pytest.mark.parametrize("N,pbc", [((16, 64, 1), (1, 0, 0)), ((24, 20, 5), (0, 1, 0)), ((10, 12, 6), (1, 1, 1)),
+                                   ((40, 14, 1), (2, 1, 0)), ((6, 40, 8), (0, 0, 1))])
+def test_periodic_lines_match_oracle(cl, N, pbc):
+    """Periodic axes (exact length, no parity split), beside open ones, and lengths without a line plan."""
+    cell = (2e-9, 2e-9, 2e-9)
+    d = cl.NewNewellDemag(N, pbc, cell)
+    m = G.random_unit(N, 8)
+    Kf, _ = O.kernel_spectrum(O.newell_kernel(N, cell, pbc))
+    want = O.demag_field(Kf, O.pad_size(N, pbc), m.astype(np.float64), 8e5, dtype=np.float64)
+    B = cu(np.zeros(m.shape, np.float32))
+    d.Exec(B, cu(m), None, 8e5)
+    assert np.abs(B.cpu().numpy() - want).max() <= 2e-6 * np.abs(want).max()
+    d.Free()

@@ -8,7 +8,8 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "libumagnus_b200.so")
 BUILD = os.path.join(HERE, "_build")
-SOURCES = ["ops.cu", "demag.cu", "demag_fast.cu", "engine.cu", "capi.cu", "noalloc.cu", "ovf.cu", "brute.cu", "adjoint.cu"]
+SOURCES = ["ops.cu", "demag.cu", "demag_fast.cu", "demag_lines_x.cu", "demag_lines_y0.cu", "demag_lines_y1.cu",
+           "demag_lines_y2.cu", "demag_lines_yp.cu", "demag_lines_z.cu", "engine.cu", "capi.cu", "noalloc.cu", "ovf.cu", "brute.cu", "adjoint.cu"]
 # per-file flags: the brute-force kernel keeps the reference's FP64 operation
 # order (no fused multiply-adds)
 FILE_FLAGS = {"brute.cu": ["-fmad=false"]}

@@ -145,7 +145,7 @@ __global__ void k_brute_mirror(double* K0, double* K1, double* K2, double* K3, d
     }
 }
 
-int build_brute(const umag_demag* d, double accuracy, double* Kr[6], cudaStream_t st) {
+int build_brute(const umag_demag* d, const int P[3], double accuracy, double* Kr[6], cudaStream_t st) {
     UMAG_REQUIRE(accuracy > 0, "demag accuracy must be positive");
     const double* c = d->cell;
     // demagkernel.go:384-398 sanityCheck: cell aspect ratio within 1/100 .. 100
@@ -154,25 +154,24 @@ int build_brute(const umag_demag* d, double accuracy, double* Kr[6], cudaStream_
     if (amax > 100.0 || amin < 1. / 100.) return set_error(UMAG_E_ARG, "unrealistic cell aspect ratio");
     BruteArgs a{};
     for (int i = 0; i < 3; i++) {
-        a.P[i] = d->P[i];
-        // kernelRanges (demagkernel.go:338-351)
+        a.P[i] = P[i];
+        // kernelRanges (demagkernel.go:338-351), whatever the padding: open axes up to N - 1
         if (d->pbc[i] == 0) { a.r1[i] = -(d->P[i] - 1) / 2; a.r2[i] = (d->P[i] - 1) / 2; }
-        else { a.r1[i] = -(d->P[i] * d->pbc[i] - 1); a.r2[i] = d->P[i] * d->pbc[i] - 1; }
+        else { a.r1[i] = -(P[i] * d->pbc[i] - 1); a.r2[i] = P[i] * d->pbc[i] - 1; }
         a.c[i] = c[i];
-        a.ext[i] = d->P[i] / 2 + 1;  // the octant [0, P/2]
+        a.ext[i] = P[i] / 2 + 1;  // the octant [0, P/2]
     }
-    if (d->P[2] == 1 && d->pbc[2] == 0) a.r2[2] = 0;
+    if (P[2] == 1 && d->pbc[2] == 0) a.r2[2] = 0;
     a.accuracy = accuracy;
     a.L = fmin(c[0], fmin(c[1], c[2]));
-    const long n = (long)d->P[0] * d->P[1] * d->P[2];
+    const long n = (long)P[0] * P[1] * P[2];
     for (int k = 0; k < 6; k++) UMAG_CUDA(cudaMemsetAsync(Kr[k], 0, sizeof(double) * n, st));
     const long npt = 3L * a.ext[0] * a.ext[1] * a.ext[2];
     k_brute_octant<<<grid_for(npt, 128, 32), 128, 0, st>>>(Kr[0], Kr[1], Kr[2], Kr[3], Kr[4], Kr[5], a);
     UMAG_LAUNCH_CHECK();
-    k_brute_mirror<<<grid_for(n, 256), 256, 0, st>>>(Kr[0], Kr[1], Kr[2], Kr[3], Kr[4], Kr[5], d->P[0], d->P[1],
-                                                      d->P[2]);
+    k_brute_mirror<<<grid_for(n, 256), 256, 0, st>>>(Kr[0], Kr[1], Kr[2], Kr[3], Kr[4], Kr[5], P[0], P[1], P[2]);
     UMAG_LAUNCH_CHECK();
-    if (d->P[2] == 1) {  // 2D: xz and yz vanish (demagkernel.go:320-324)
+    if (P[2] == 1) {  // 2D: xz and yz vanish (demagkernel.go:320-324)
         UMAG_CUDA(cudaMemsetAsync(Kr[3], 0, sizeof(double) * n, st));
         UMAG_CUDA(cudaMemsetAsync(Kr[4], 0, sizeof(double) * n, st));
     }

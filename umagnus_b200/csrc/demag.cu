@@ -436,6 +436,7 @@ static size_t pass_ac_smem(const umag_demag* d) {
     return sizeof(float2) * ((size_t)d->N[2] * d->HxP + (d->P[2] > 1 ? (size_t)d->P[2] * kChunkW : 0));
 }
 static size_t pass_b_smem(const umag_demag* d) { return sizeof(float2) * (size_t)d->P[1] * 3 * d->WB; }
+static size_t spec_elems(const umag_demag* d) { return (size_t)3 * d->F[2] * d->N[1] * d->Lx; }
 
 // Tensor map for pass C's slab loads (PassArgs::slab_map): the blocked
 // spectrum as floats (8 = four complex columns, y, kx/4, kz, component), a
@@ -443,9 +444,9 @@ static size_t pass_b_smem(const umag_demag* d) { return sizeof(float2) * (size_t
 // slab shape and the slab fits the x/z scratch it borrows.  Without it pass C
 // keeps its plain loads.
 static void slab_setup(umag_demag* d) {
-    const FastPasses& f = d->fast;
-    if (!d->use_fast || !f.blocked || !f.slab_ok || d->Lx % 4 != 0) return;
-    const int KB = d->Lx / 4, Ny = d->N[1], Pz = d->P[2];
+    const Passes& f = d->fast;
+    if (!d->use_lines || !f.a || !f.slab_ok || d->Lx % 4 != 0) return;
+    const int KB = d->Lx / 4, Ny = d->N[1], Pz = d->F[2];
     const size_t bytes = sizeof(float2) * 4 * (size_t)KB * Pz;
     if (bytes + 128 > f.ac_scratch || KB > 256 || Pz > 256) return;  // + the alignment slack
     EncodeTiledFn fn = encode_tiled();
@@ -470,7 +471,9 @@ static void slab_setup(umag_demag* d) {
     d->slab_map = dev;
 }
 
-static int plan_common(umag_demag* d) {
+// Checks of the reference sizes (what the plan accepts does not depend on the
+// passes that then run it) and the pass-B block of the runtime-planned passes.
+static int plan_check(umag_demag* d) {
     for (int i = 0; i < 3; i++) UMAG_REQUIRE(d->N[i] > 0, "mesh size must be positive");
     for (int i = 0; i < 3; i++) UMAG_REQUIRE(d->pbc[i] >= 0, "PBC repetitions must be non-negative");
     // mag/demagkernel.go:404-420: no padding along a periodic axis
@@ -479,17 +482,17 @@ static int plan_common(umag_demag* d) {
     d->P[2] = d->pbc[2] ? d->N[2] : (d->N[2] > 5 ? 2 * d->N[2] : 2 * d->N[2] - 1);
     if (d->P[0] % 2 != 0)
         return set_error(UMAG_E_UNSUPPORTED, "periodic x needs an even Nx (the x transform packs pairs of reals)");
-    d->M = d->P[0] / 2;
-    d->Hx = d->M + 1;
-    d->HxP = d->M + 1;
-    d->Lx = (d->Hx + 3) / 4 * 4;
+    d->HxP = d->P[0] / 2 + 1;
     d->is2d = d->N[2] == 1;
+    FftLine<float> fl[3];
+    const int len[3] = {d->P[0] / 2, d->P[1], d->P[2]};
+    for (int i = 0; i < 3; i++) {
+        fl[i].L = len[i];
+        fl[i].nst = len[i] > 1 ? fft_factor(len[i], fl[i].R) : 0;
+    }
     // pass B column block: 3*WB*Py elements must fit the register capacity
     int wb = 8;
-    FftLine<float> probe{};
-    probe.L = d->P[1];
-    probe.nst = fft_factor(d->P[1], probe.R);
-    int capy = fft_line_cap(probe);
+    const int capy = fft_line_cap(fl[1]);
     while (wb > 1 && 3 * wb * d->P[1] > kPassBThreads * capy) wb /= 2;
     if (3 * wb * d->P[1] > kPassBThreads * capy)
         return set_error(UMAG_E_UNSUPPORTED, "padded Ny = %d too large for pass B", d->P[1]);
@@ -498,49 +501,56 @@ static int plan_common(umag_demag* d) {
         return set_error(UMAG_E_UNSUPPORTED, "Nz*(Nx+1) too large for the x/z passes (%zu bytes smem)",
                          pass_ac_smem(d));
     if (pass_b_smem(d) > 227 * 1024) return set_error(UMAG_E_UNSUPPORTED, "pass B shared memory too large");
+    for (int i = 0; i < 3; i++)
+        if (!fft_max_radix_ok(fl[i].R, fl[i].nst))
+            return set_error(UMAG_E_UNSUPPORTED, "FFT length %d has a prime factor above 13", len[i]);
+    if (!fft_line_fits(fl[0], kPassThreads))
+        return set_error(UMAG_E_UNSUPPORTED, "Nx = %d too large for the x pass", d->N[0]);
+    if (d->P[2] > 1 && (long)kChunkW * d->P[2] > (long)kPassThreads * fft_line_cap(fl[2]))
+        return set_error(UMAG_E_UNSUPPORTED, "Nz = %d too large for the z transform", d->N[2]);
+    return UMAG_OK;
+}
+
+static int plan_common(umag_demag* d) {
+    UMAG_TRY(plan_check(d));
+    d->use_lines = getenv("UMAG_GENERIC_FFT") == nullptr && lines_select(d->N, d->pbc, d->F, d->fast, false);
+    if (!d->use_lines)
+        for (int i = 0; i < 3; i++) d->F[i] = d->P[i];
+    d->M = d->F[0] / 2;
+    d->Hx = d->M + 1;
+    d->Lx = (d->Hx + 3) / 4 * 4;
     float2* tw;
     UMAG_TRY(make_line<float>(d->M, d->fx, &tw)); d->tw_dev.push_back(tw);
-    UMAG_TRY(make_line<float>(d->P[1], d->fy, &tw)); d->tw_dev.push_back(tw);
-    UMAG_TRY(make_line<float>(d->P[2], d->fz, &tw)); d->tw_dev.push_back(tw);
-    if (!fft_line_fits(d->fx, kPassThreads))
-        return set_error(UMAG_E_UNSUPPORTED, "Nx = %d too large for the x pass", d->N[0]);
-    if (d->P[2] > 1 && (long)kChunkW * d->P[2] > (long)kPassThreads * fft_line_cap(d->fz))
-        return set_error(UMAG_E_UNSUPPORTED, "Nz = %d too large for the z transform", d->N[2]);
-    auto twr = twiddles<float2>(d->P[0], d->M > 1 ? d->M : 2);  // exp(-2 pi i k / Px), k < Px/2
+    UMAG_TRY(make_line<float>(d->F[1], d->fy, &tw)); d->tw_dev.push_back(tw);
+    UMAG_TRY(make_line<float>(d->F[2], d->fz, &tw)); d->tw_dev.push_back(tw);
+    auto twr = twiddles<float2>(d->F[0], d->M > 1 ? d->M : 2);  // exp(-2 pi i k / Px), k < Px/2
     UMAG_CUDA(cudaMalloc(&d->twr, sizeof(float2) * twr.size()));
     UMAG_CUDA(cudaMemcpyAsync(d->twr, twr.data(), sizeof(float2) * twr.size(), cudaMemcpyHostToDevice, ctx().stream));
     UMAG_CUDA(cudaStreamSynchronize(ctx().stream));
-    size_t spec_elems = (size_t)3 * d->P[2] * d->N[1] * d->Lx;
-    UMAG_CUDA(cudaMalloc(&d->spec, sizeof(float2) * spec_elems));
-    UMAG_CUDA(cudaMemsetAsync(d->spec, 0, sizeof(float2) * spec_elems, ctx().stream));
+    UMAG_CUDA(cudaMalloc(&d->spec, sizeof(float2) * spec_elems(d)));
+    UMAG_CUDA(cudaMemsetAsync(d->spec, 0, sizeof(float2) * spec_elems(d), ctx().stream));
     d->Kp = (d->Hx + 3) / 4 * 4;
-    size_t kn = (size_t)d->Kp * (d->P[1] / 2 + 1) * (d->P[2] / 2 + 1);
+    size_t kn = (size_t)d->Kp * (d->F[1] / 2 + 1) * (d->F[2] / 2 + 1);
     d->Kn = kn;
     for (int c = 0; c < 6; c++) {
         d->K[c] = nullptr;
         if (d->is2d && (c == 3 || c == 4)) continue;  // yz, xz vanish in 2D (newellDemagKernel.go:1314-1317)
         UMAG_CUDA(cudaMalloc(&d->K[c], sizeof(float) * kn));
     }
-    // the opt-in limit is per kernel and process-wide: set it to the maximum
-    // so plans of different sizes can coexist
-    const int maxsm = 227 * 1024;
-    UMAG_CUDA(cudaFuncSetAttribute(k_pass_a, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsm));
-    UMAG_CUDA(cudaFuncSetAttribute(k_pass_c, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsm));
-    UMAG_CUDA(cudaFuncSetAttribute(k_pass_b, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsm));
-    UMAG_CUDA(cudaFuncSetAttribute(k_fft_axis<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsm));
-    UMAG_TRY(demag_fast_setup());
-    // the compile-time passes assume a zero-padded half along x and y
-    const bool periodic = d->pbc[0] || d->pbc[1] || d->pbc[2];
-    d->use_fast = !periodic && getenv("UMAG_GENERIC_FFT") == nullptr &&
-                  demag_fast_select(d->M, d->P[1], d->P[2], d->fast);
-    if (d->use_fast) UMAG_TRY(demag_fast_grid(d->fast, d->M, d->P[2]));
+    UMAG_TRY(passes_attrs(d->fast));
+    UMAG_TRY(pass_attrs(k_pass_a));
+    UMAG_TRY(pass_attrs(k_pass_b));
+    UMAG_TRY(pass_attrs(k_pass_c));
+    UMAG_CUDA(cudaFuncSetAttribute(k_fft_axis<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     slab_setup(d);
     return UMAG_OK;
 }
 
 // FP64 real-space kernel -> float32 spectrum (opencl/conv_demag.go:155-201)
-static int kernel_to_spectrum(umag_demag* d, double* const Kr[6], cudaStream_t st) {
-    const int Px = d->P[0], Py = d->P[1], Pz = d->P[2];
+// of size P, rows of Kp floats or 4-column blocks, into the arrays K that exist
+static int kernel_to_spectrum(const int P[3], double* const Kr[6], float* const K[6], int Kp, int blocked,
+                              cudaStream_t st) {
+    const int Px = P[0], Py = P[1], Pz = P[2];
     long n = (long)Px * Py * Pz;
     double2* buf = nullptr;
     UMAG_CUDA(cudaMalloc(&buf, sizeof(double2) * n));
@@ -548,18 +558,18 @@ static int kernel_to_spectrum(umag_demag* d, double* const Kr[6], cudaStream_t s
     double2* tws[3] = {nullptr, nullptr, nullptr};
     int st_ok = UMAG_OK;
     for (int ax = 0; ax < 3 && st_ok == UMAG_OK; ax++) {
-        st_ok = make_line<double>(d->P[ax], fl[ax], &tws[ax]);
+        st_ok = make_line<double>(P[ax], fl[ax], &tws[ax]);
         if (st_ok == UMAG_OK && !fft_line_fits(fl[ax], 256))
-            st_ok = set_error(UMAG_E_UNSUPPORTED, "kernel FFT line %d too long", d->P[ax]);
+            st_ok = set_error(UMAG_E_UNSUPPORTED, "kernel FFT line %d too long", P[ax]);
     }
     unsigned long long* dmax = nullptr;
     if (st_ok == UMAG_OK) st_ok = cudaMalloc(&dmax, sizeof(unsigned long long)) == cudaSuccess ? UMAG_OK : UMAG_E_CUDA;
     const int threads = 256;
     for (int c = 0; c < 6 && st_ok == UMAG_OK; c++) {
-        if (d->K[c] == nullptr) continue;
+        if (K[c] == nullptr) continue;
         k_real_to_cplx<<<grid_for(n, threads), threads, 0, st>>>(Kr[c], buf, n);
         for (int ax = 0; ax < 3; ax++) {
-            int L = d->P[ax];
+            int L = P[ax];
             if (L == 1) continue;
             int G = ax == 0 ? 1 : 4;
             while (ax == 0 && (G * 2) * L * 16 <= 64 * 1024 && G < 8) G *= 2;
@@ -571,10 +581,9 @@ static int kernel_to_spectrum(umag_demag* d, double* const Kr[6], cudaStream_t s
             k_fft_axis<double><<<(unsigned)blocks, threads, sm, st>>>(buf, fl[ax], Px, Py, Pz, ax, G, -1);
         }
         cudaMemsetAsync(dmax, 0, sizeof(unsigned long long), st);
-        long kn = (long)d->Kn;
-        k_extract_spectrum<<<grid_for(kn, threads), threads, 0, st>>>(buf, d->K[c], Px, Py, Pz, d->Kp,
-                                                                       d->use_fast && d->fast.blocked ? 1 : 0,
-                                                                       1.0 / (double)n, dmax);
+        long kn = (long)Kp * (Py / 2 + 1) * (Pz / 2 + 1);
+        k_extract_spectrum<<<grid_for(kn, threads), threads, 0, st>>>(buf, K[c], Px, Py, Pz, Kp, blocked, 1.0 / (double)n,
+                                                                       dmax);
         unsigned long long hm = 0;
         cudaMemcpyAsync(&hm, dmax, sizeof(hm), cudaMemcpyDeviceToHost, st);
         if (cudaStreamSynchronize(st) != cudaSuccess) { st_ok = set_error(UMAG_E_CUDA, "kernel FFT failed"); break; }
@@ -591,17 +600,17 @@ static int kernel_to_spectrum(umag_demag* d, double* const Kr[6], cudaStream_t s
 }
 
 // Newell tensor in FP64 on the device (mag/newellDemagKernel.go:1108-1324)
-static int build_newell(const umag_demag* d, const double cell[3], int arad, int zero_self, double* Kr[6],
-                        cudaStream_t st) {
+static int build_newell(const umag_demag* d, const int P[3], const double cell[3], int arad, int zero_self,
+                        double* Kr[6], cudaStream_t st) {
     NewellArgs a{};
     for (int i = 0; i < 3; i++) {
-        a.P[i] = d->P[i];
-        a.ext[i] = d->P[i] / 2 + 1;  // octant [0, P/2]
-        // kernelRanges (mag/demagkernel.go:339-352)
+        a.P[i] = P[i];
+        a.ext[i] = P[i] / 2 + 1;  // octant [0, P/2]
+        // kernelRanges (mag/demagkernel.go:339-352), whatever the padding: open axes up to N - 1
         if (d->pbc[i] == 0) { a.r1[i] = -(d->P[i] - 1) / 2; a.r2[i] = (d->P[i] - 1) / 2; }
-        else { a.r1[i] = -(d->P[i] * d->pbc[i] - 1); a.r2[i] = d->P[i] * d->pbc[i] - 1; }
+        else { a.r1[i] = -(P[i] * d->pbc[i] - 1); a.r2[i] = P[i] * d->pbc[i] - 1; }
     }
-    if (d->P[2] == 1 && d->pbc[2] == 0) a.r2[2] = 0;
+    if (P[2] == 1 && d->pbc[2] == 0) a.r2[2] = 0;
     double dx = cell[0], dy = cell[1], dz = cell[2];
     newell::reduce_cell(dx, dy, dz);
     a.dx = dx; a.dy = dy; a.dz = dz;
@@ -615,24 +624,58 @@ static int build_newell(const umag_demag* d, const double cell[3], int arad, int
     a.eyy = newell::make_expansion(0, dy, dx, dz);
     a.eyz = newell::make_expansion(1, dy, dz, dx);
     a.ezz = newell::make_expansion(0, dz, dy, dx);
-    long n = (long)d->P[0] * d->P[1] * d->P[2];
+    long n = (long)P[0] * P[1] * P[2];
     for (int c = 0; c < 6; c++) UMAG_CUDA(cudaMemsetAsync(Kr[c], 0, sizeof(double) * n, st));
     long oct = (long)a.ext[0] * a.ext[1] * a.ext[2];
     k_newell_octant<<<grid_for(oct, 128, 32), 128, 0, st>>>(Kr[0], Kr[1], Kr[2], Kr[3], Kr[4], Kr[5], a);
     UMAG_LAUNCH_CHECK();
-    k_newell_mirror<<<grid_for(n, 256), 256, 0, st>>>(Kr[0], Kr[1], Kr[2], Kr[3], Kr[4], Kr[5], d->P[0], d->P[1],
-                                                       d->P[2]);
+    k_newell_mirror<<<grid_for(n, 256), 256, 0, st>>>(Kr[0], Kr[1], Kr[2], Kr[3], Kr[4], Kr[5], P[0], P[1],
+                                                       P[2]);
     UMAG_LAUNCH_CHECK();
     // self terms at the origin (:1300-1312)
     double self[6] = {-newell::self_nx(dx, dy, dz), -newell::self_nx(dy, dz, dx), -newell::self_nx(dz, dx, dy),
                       0.0, 0.0, 0.0};
     if (zero_self) for (int c = 0; c < 3; c++) self[c] += 1.0 / 3.0;
     for (int c = 0; c < 6; c++) UMAG_CUDA(cudaMemcpyAsync(Kr[c], &self[c], sizeof(double), cudaMemcpyHostToDevice, st));
-    if (d->P[2] == 1) {
+    if (P[2] == 1) {
         UMAG_CUDA(cudaMemsetAsync(Kr[3], 0, sizeof(double) * n, st));
         UMAG_CUDA(cudaMemsetAsync(Kr[4], 0, sizeof(double) * n, st));
     }
     UMAG_CUDA(cudaStreamSynchronize(st));
+    return UMAG_OK;
+}
+
+// six zeroed or filled device arrays of a padded grid P
+struct KernelGrid {
+    double* K[6] = {};
+    long n = 0;
+    int alloc(const int P[3]) {
+        n = (long)P[0] * P[1] * P[2];
+        for (int c = 0; c < 6; c++)
+            if (cudaMalloc(&K[c], sizeof(double) * n) != cudaSuccess) return set_error(UMAG_E_NOMEM, "kernel buffers");
+        return UMAG_OK;
+    }
+    ~KernelGrid() {
+        for (int c = 0; c < 6; c++) cudaFree(K[c]);
+    }
+};
+
+// the plan's real-space kernel on the grid P (kinds 0 and 1)
+static int build_kernel(const umag_demag* d, const int P[3], double* Kr[6], cudaStream_t st) {
+    if (d->kind == 0) return build_newell(d, P, d->cell, d->arad, d->zero_self, Kr, st);
+    return build_brute(d, P, d->accuracy, Kr, st);
+}
+
+static int plan_new(umag_demag* d, umag_demag** out) {
+    int s = plan_common(d);
+    if (s == UMAG_OK) {
+        KernelGrid g;
+        s = g.alloc(d->F);
+        if (s == UMAG_OK) s = build_kernel(d, d->F, g.K, ctx().stream);
+        if (s == UMAG_OK) s = kernel_to_spectrum(d->F, g.K, d->K, d->Kp, d->use_lines ? 1 : 0, ctx().stream);
+    }
+    if (s != UMAG_OK) { demag_free(d); return s; }
+    *out = d;
     return UMAG_OK;
 }
 
@@ -647,19 +690,7 @@ int demag_new_newell(int Nx, int Ny, int Nz, const int pbc[3], double cx, double
     d->arad = arad;
     d->zero_self = zero_self;
     for (int i = 0; i < 3; i++) d->pbc[i] = pbc ? pbc[i] : 0;
-    int s = plan_common(d);
-    if (s != UMAG_OK) { demag_free(d); return s; }
-    cudaStream_t st = ctx().stream;
-    long n = (long)d->P[0] * d->P[1] * d->P[2];
-    double* Kr[6] = {};
-    for (int c = 0; c < 6 && s == UMAG_OK; c++)
-        if (cudaMalloc(&Kr[c], sizeof(double) * n) != cudaSuccess) s = set_error(UMAG_E_NOMEM, "kernel buffers");
-    if (s == UMAG_OK) s = build_newell(d, d->cell, arad, zero_self, Kr, st);
-    if (s == UMAG_OK) s = kernel_to_spectrum(d, Kr, st);
-    for (int c = 0; c < 6; c++) cudaFree(Kr[c]);
-    if (s != UMAG_OK) { demag_free(d); return s; }
-    *out = d;
-    return UMAG_OK;
+    return plan_new(d, out);
 }
 
 // mag/demagkernel.go:113 CalcDemagKernel (engine/demag.go:124-133 demagConv):
@@ -676,20 +707,45 @@ int demag_new_brute(int Nx, int Ny, int Nz, const int pbc[3], double cx, double 
     d->kind = 1;
     d->accuracy = accuracy;
     for (int i = 0; i < 3; i++) d->pbc[i] = pbc ? pbc[i] : 0;
-    int s = plan_common(d);
-    if (s != UMAG_OK) { demag_free(d); return s; }
-    cudaStream_t st = ctx().stream;
-    long n = (long)d->P[0] * d->P[1] * d->P[2];
-    double* Kr[6] = {};
-    for (int c = 0; c < 6 && s == UMAG_OK; c++)
-        if (cudaMalloc(&Kr[c], sizeof(double) * n) != cudaSuccess) s = set_error(UMAG_E_NOMEM, "kernel buffers");
-    if (s == UMAG_OK) s = build_brute(d, accuracy, Kr, st);
-    if (s == UMAG_OK) s = kernel_to_spectrum(d, Kr, st);
-    for (int c = 0; c < 6; c++) cudaFree(Kr[c]);
-    if (s != UMAG_OK) { demag_free(d); return s; }
-    *out = d;
-    return UMAG_OK;
+    return plan_new(d, out);
 }
+
+// A caller's kernel on the padded grid P moved to the grid F: offsets up to
+// N - 1 each way are all that the field of the mesh depends on.
+__global__ void k_repad_kernel(const double* __restrict__ src, double* __restrict__ dst, int Nx, int Ny, int Nz, int Px,
+                               int Py, int Pz, int Fx, int Fy, int Fz) {
+    const long n = (long)Fx * Fy * Fz;
+    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
+        const int x = (int)(i % Fx), y = (int)((i / Fx) % Fy), z = (int)(i / ((long)Fx * Fy));
+        const int ox = x < Nx ? x : x - Fx, oy = y < Ny ? y : y - Fy, oz = z < Nz ? z : z - Fz;
+        double v = 0.0;
+        if (ox > -Nx && oy > -Ny && oz > -Nz)
+            v = src[((long)(oz < 0 ? oz + Pz : oz) * Py + (oy < 0 ? oy + Py : oy)) * Px + (ox < 0 ? ox + Px : ox)];
+        dst[i] = v;
+    }
+}
+
+// the spectrum on the reference's padded sizes in its layout (rows of
+// P[0]/2+1 floats), to the host
+static int reference_spectrum(umag_demag* d, double* const Kr[6], std::vector<float> out[6]) {
+    const int Kp = d->P[0] / 2 + 1;
+    const size_t kn = (size_t)Kp * (d->P[1] / 2 + 1) * (d->P[2] / 2 + 1);
+    float* K[6] = {};
+    int s = UMAG_OK;
+    for (int c = 0; c < 6 && s == UMAG_OK; c++)
+        if (d->K[c] && cudaMalloc(&K[c], sizeof(float) * kn) != cudaSuccess) s = set_error(UMAG_E_NOMEM, "spectrum");
+    if (s == UMAG_OK) s = kernel_to_spectrum(d->P, Kr, K, Kp, 0, ctx().stream);
+    for (int c = 0; c < 6 && s == UMAG_OK; c++) {
+        if (!K[c]) continue;
+        out[c].resize(kn);
+        if (cudaMemcpyAsync(out[c].data(), K[c], sizeof(float) * kn, cudaMemcpyDeviceToHost, ctx().stream) != cudaSuccess ||
+            cudaStreamSynchronize(ctx().stream) != cudaSuccess)
+            s = set_error(UMAG_E_CUDA, "copy spectrum");
+    }
+    for (int c = 0; c < 6; c++) cudaFree(K[c]);
+    return s;
+}
+
 int demag_new_from_kernel(int Nx, int Ny, int Nz, const double* const kern[6], umag_demag** out) {
     UMAG_TRY(ensure_init());
     UMAG_REQUIRE(out != nullptr && kern != nullptr, "NULL argument");
@@ -698,17 +754,30 @@ int demag_new_from_kernel(int Nx, int Ny, int Nz, const double* const kern[6], u
     d->kind = 2;
     int s = plan_common(d);
     if (s != UMAG_OK) { demag_free(d); return s; }
-    long n = (long)d->P[0] * d->P[1] * d->P[2];
-    double* Kr[6] = {};
-    for (int c = 0; c < 6 && s == UMAG_OK; c++) {
-        if (cudaMalloc(&Kr[c], sizeof(double) * n) != cudaSuccess) { s = set_error(UMAG_E_NOMEM, "kernel"); break; }
-        const cudaError_t e = kern[c] ? cudaMemcpyAsync(Kr[c], kern[c], sizeof(double) * n, cudaMemcpyHostToDevice,
-                                                        ctx().stream)
-                                      : cudaMemsetAsync(Kr[c], 0, sizeof(double) * n, ctx().stream);
-        if (e != cudaSuccess) s = set_error(UMAG_E_CUDA, "kernel upload: %s", cudaGetErrorString(e));
+    const int *P = d->P, *F = d->F;
+    {
+        KernelGrid g, h;
+        s = g.alloc(P);
+        for (int c = 0; c < 6 && s == UMAG_OK; c++) {
+            const cudaError_t e = kern[c] ? cudaMemcpyAsync(g.K[c], kern[c], sizeof(double) * g.n,
+                                                            cudaMemcpyHostToDevice, ctx().stream)
+                                          : cudaMemsetAsync(g.K[c], 0, sizeof(double) * g.n, ctx().stream);
+            if (e != cudaSuccess) s = set_error(UMAG_E_CUDA, "kernel upload: %s", cudaGetErrorString(e));
+        }
+        const bool same = F[0] == P[0] && F[1] == P[1] && F[2] == P[2];
+        if (s == UMAG_OK && !same) {
+            // the caller's grid is checked and reported as given; the passes use the other
+            s = reference_spectrum(d, g.K, d->ref_spec);
+            if (s == UMAG_OK) s = h.alloc(F);
+            for (int c = 0; c < 6 && s == UMAG_OK; c++) {
+                k_repad_kernel<<<grid_for(h.n, 256), 256, 0, ctx().stream>>>(g.K[c], h.K[c], Nx, Ny, Nz, P[0], P[1],
+                                                                             P[2], F[0], F[1], F[2]);
+                if (cudaGetLastError() != cudaSuccess) s = set_error(UMAG_E_CUDA, "kernel padding");
+            }
+        }
+        if (s == UMAG_OK)
+            s = kernel_to_spectrum(F, same ? g.K : h.K, d->K, d->Kp, d->use_lines ? 1 : 0, ctx().stream);
     }
-    if (s == UMAG_OK) s = kernel_to_spectrum(d, Kr, ctx().stream);
-    for (int c = 0; c < 6; c++) cudaFree(Kr[c]);
     if (s != UMAG_OK) { demag_free(d); return s; }
     *out = d;
     return UMAG_OK;
@@ -722,8 +791,7 @@ int demag_get_kernel(umag_demag* d, double* const host[6]) {
     for (int c = 0; c < 6 && s == UMAG_OK; c++)
         if (cudaMalloc(&Kr[c], sizeof(double) * n) != cudaSuccess) s = set_error(UMAG_E_NOMEM, "kernel buffers");
     if (s == UMAG_OK) {
-        if (d->kind == 0) s = build_newell(d, d->cell, d->arad, d->zero_self, Kr, ctx().stream);
-        else if (d->kind == 1) s = build_brute(d, d->accuracy, Kr, ctx().stream);
+        if (d->kind != 2) s = build_kernel(d, d->P, Kr, ctx().stream);
         else s = set_error(UMAG_E_UNSUPPORTED, "the plan was built from a caller-supplied kernel, which it does not keep");
     }
     for (int c = 0; c < 6 && s == UMAG_OK; c++)
@@ -738,17 +806,29 @@ int demag_get_kernel(umag_demag* d, double* const host[6]) {
 int demag_get_spectrum(umag_demag* d, float* const host[6]) {
     UMAG_REQUIRE(d != nullptr, "NULL plan");
     UMAG_CUDA(cudaStreamSynchronize(ctx().stream));
-    const size_t hy = d->P[1] / 2 + 1, rows = d->Kn / d->Kp;  // rows = hy * hz
-    const bool blocked = d->use_fast && d->fast.blocked;
-    std::vector<float> tmp(blocked ? d->Kn : 0);
+    const size_t hx = d->P[0] / 2 + 1, hy = d->P[1] / 2 + 1, rows = hy * (d->P[2] / 2 + 1);
+    const bool same = d->F[0] == d->P[0] && d->F[1] == d->P[1] && d->F[2] == d->P[2];
+    std::vector<float> built[6], *ref = nullptr;
+    if (!same && d->kind == 2) {
+        ref = d->ref_spec;
+    } else if (!same) {
+        KernelGrid g;
+        UMAG_TRY(g.alloc(d->P));
+        UMAG_TRY(build_kernel(d, d->P, g.K, ctx().stream));
+        UMAG_TRY(reference_spectrum(d, g.K, built));
+        ref = built;
+    }
+    std::vector<float> tmp(d->use_lines && same ? d->Kn : 0);
     for (int c = 0; c < 6; c++) {
         if (!host[c]) continue;
         if (!d->K[c]) {
-            memset(host[c], 0, sizeof(float) * d->Hx * rows);
-        } else if (!blocked) {
+            memset(host[c], 0, sizeof(float) * hx * rows);
+        } else if (ref) {
+            memcpy(host[c], ref[c].data(), sizeof(float) * hx * rows);
+        } else if (!d->use_lines) {
             // reference layout: rows of Px/2+1 floats (the device rows are padded to Kp)
-            UMAG_CUDA(cudaMemcpy2DAsync(host[c], sizeof(float) * d->Hx, d->K[c], sizeof(float) * d->Kp,
-                                        sizeof(float) * d->Hx, rows, cudaMemcpyDeviceToHost, ctx().stream));
+            UMAG_CUDA(cudaMemcpy2DAsync(host[c], sizeof(float) * hx, d->K[c], sizeof(float) * d->Kp,
+                                        sizeof(float) * hx, rows, cudaMemcpyDeviceToHost, ctx().stream));
             UMAG_CUDA(cudaStreamSynchronize(ctx().stream));
         } else {
             UMAG_CUDA(cudaMemcpyAsync(tmp.data(), d->K[c], sizeof(float) * d->Kn, cudaMemcpyDeviceToHost, ctx().stream));
@@ -756,8 +836,7 @@ int demag_get_spectrum(umag_demag* d, float* const host[6]) {
             const size_t nb = d->Kp / 4;
             for (size_t r = 0; r < rows; r++) {  // r = z * hy + y
                 const size_t z = r / hy, y = r % hy;
-                for (int x = 0; x < d->Hx; x++)
-                    host[c][r * d->Hx + x] = tmp[((z * nb + x / 4) * hy + y) * 4 + x % 4];
+                for (size_t x = 0; x < hx; x++) host[c][r * hx + x] = tmp[((z * nb + x / 4) * hy + y) * 4 + x % 4];
             }
         }
     }
@@ -766,73 +845,72 @@ int demag_get_spectrum(umag_demag* d, float* const host[6]) {
 
 void fill_pass_args(const umag_demag* d, PassArgs& a) {
     a.Nx = d->N[0]; a.Ny = d->N[1]; a.Nz = d->N[2];
-    a.Px = d->P[0]; a.Py = d->P[1]; a.Pz = d->P[2];
+    a.Px = d->F[0]; a.Py = d->F[1]; a.Pz = d->F[2];
     a.M = d->M; a.Hx = d->Hx; a.HxP = d->HxP; a.Lx = d->Lx; a.WB = d->WB;
     a.fx = d->fx; a.fy = d->fy; a.fz = d->fz;
     a.twr = d->twr;
     a.spec = d->spec;
     for (int c = 0; c < 6; c++) a.K[c] = d->K[c];
     a.Kp = d->Kp;
-    a.blocked = d->use_fast && d->fast.blocked ? 1 : 0;
-    a.Kblocked = a.blocked;
+    a.Kblocked = d->use_lines ? 1 : 0;
     a.slab_map = d->slab_map;
+    demag_timeouts_ptr(&a.timeouts);
 }
 
-int demag_launch(const umag_demag* d, const PassArgs& a, cudaStream_t st) {
-    if (d->use_fast) {
-        const FastPasses& f = d->fast;
-        f.a<<<dim3(d->N[1], 3), f.nt_ac, f.smem_ac, st>>>(a);
-        UMAG_LAUNCH_CHECK();
-        if (f.use_narrow) f.b_n<<<dim3(f.gbx_n, f.gby), f.nt_b_n, f.smem_b_n, st>>>(a);
-        else f.b<<<dim3(f.gbx, f.gby), f.nt_b, f.smem_b, st>>>(a);
-        UMAG_LAUNCH_CHECK();
-        f.c<<<dim3(d->N[1], 3), f.nt_ac, f.smem_ac, st>>>(a);
+// pass 0: scaled m to the spectrum (x, z), 1: y and the kernel, 2: back to B,
+// for nb instances at once
+static int launch_pass(const umag_demag* d, const PassArgs& a, int nb, int pass, cudaStream_t st) {
+    const int Nx3 = 3 * d->N[2], Ny = d->N[1];
+    if (!d->use_lines) {
+        const size_t sac = pass_ac_smem(d), sb = pass_b_smem(d);
+        if (pass == 0) k_pass_a<<<dim3(Ny, 3), kPassThreads, sac, st>>>(a);
+        else if (pass == 1) k_pass_b<<<dim3((d->Hx + d->WB - 1) / d->WB, d->P[2]), kPassBThreads, sb, st>>>(a);
+        else k_pass_c<<<dim3(Ny, 3), kPassThreads, sac, st>>>(a);
         UMAG_LAUNCH_CHECK();
         return UMAG_OK;
     }
-    size_t sac = pass_ac_smem(d), sb = pass_b_smem(d);
-    k_pass_a<<<dim3(d->N[1], 3), kPassThreads, sac, st>>>(a);
-    UMAG_LAUNCH_CHECK();
-    k_pass_b<<<dim3((d->Hx + d->WB - 1) / d->WB, d->P[2]), kPassBThreads, sb, st>>>(a);
-    UMAG_LAUNCH_CHECK();
-    k_pass_c<<<dim3(d->N[1], 3), kPassThreads, sac, st>>>(a);
+    const Passes& f = d->fast;
+    if (pass == 1) {
+        f.y<<<dim3(d->Lx / 4, d->F[2], nb), f.nt_y, d->is2d ? f.smem_y2 : f.smem_y3, st>>>(a);
+    } else if (f.a) {
+        if (pass == 0) (nb > 1 ? f.ab : f.a)<<<dim3(Ny, 3 * nb), f.nt_ac, f.smem_ac, st>>>(a);
+        else (nb > 1 ? f.cb : f.c)<<<dim3(Ny, 3 * nb), f.nt_ac, f.smem_ac, st>>>(a);
+    } else {
+        const dim3 gx((Ny + 3) / 4, Nx3, nb), gz((unsigned)(((long)Ny * d->Lx + 127) / 128), 3, nb);
+        if (pass == 0) {
+            f.xf<<<gx, f.nt_x, f.smem_x, st>>>(a);
+            UMAG_LAUNCH_CHECK();
+            if (f.zf) f.zf<<<gz, 128, 0, st>>>(a);
+        } else {
+            if (f.zi) f.zi<<<gz, 128, 0, st>>>(a);
+            UMAG_LAUNCH_CHECK();
+            f.xi<<<gx, f.nt_x, f.smem_x, st>>>(a);
+        }
+    }
     UMAG_LAUNCH_CHECK();
     return UMAG_OK;
 }
 
-// the three passes for nb same-size instances at once (batched kernels; the
-// per-instance pointers are shifted by the strides in PassArgs)
+int demag_launch(const umag_demag* d, const PassArgs& a, cudaStream_t st) {
+    for (int pass = 0; pass < 3; pass++) UMAG_TRY(launch_pass(d, a, 1, pass, st));
+    return UMAG_OK;
+}
+
+// kernels one demag_launch queues
+int demag_launches(const umag_demag* d) {
+    if (!d->use_lines || d->fast.a || !d->fast.zf) return 3;
+    return 5;
+}
+
+// the passes for nb same-size instances at once (the per-instance pointers
+// are shifted by the strides in PassArgs)
 int demag_launch_batch(const umag_demag* d, const PassArgs& a, int nb, cudaStream_t st) {
-    UMAG_REQUIRE(d->use_fast && d->fast.ab && d->fast.bb && d->fast.cb, "batched demag needs a compile-time FFT plan");
-    UMAG_REQUIRE(nb >= 1 && 3L * nb <= 65535 && (long)d->fast.gby * nb <= 65535, "too many instances in one batch");
-    const FastPasses& f = d->fast;
+    UMAG_REQUIRE(d->use_lines && listed_mesh(d->N, d->P), "batched demag needs a compile-time FFT plan");
+    UMAG_REQUIRE(nb >= 1 && 3L * nb <= 65535 && (long)d->F[2] * nb <= 65535, "too many instances in one batch");
     // per-instance spectra: the slab map covers the plan's own spectrum only
     PassArgs ab = a;
     ab.slab_map = nullptr;
-    f.ab<<<dim3(d->N[1], 3 * nb), f.nt_ac, f.smem_ac, st>>>(ab);
-    UMAG_LAUNCH_CHECK();
-    f.bb<<<dim3(f.gbx, f.gby * nb), f.nt_b, f.smem_b, st>>>(ab);
-    UMAG_LAUNCH_CHECK();
-    f.cb<<<dim3(d->N[1], 3 * nb), f.nt_ac, f.smem_ac, st>>>(ab);
-    UMAG_LAUNCH_CHECK();
-    return UMAG_OK;
-}
-
-// one pass of demag_launch (0: A, 1: B, 2: C)
-static int demag_launch_pass(const umag_demag* d, const PassArgs& a, cudaStream_t st, int pass) {
-    if (d->use_fast) {
-        const FastPasses& f = d->fast;
-        if (pass == 0) f.a<<<dim3(d->N[1], 3), f.nt_ac, f.smem_ac, st>>>(a);
-        else if (pass == 1 && f.use_narrow) f.b_n<<<dim3(f.gbx_n, f.gby), f.nt_b_n, f.smem_b_n, st>>>(a);
-        else if (pass == 1) f.b<<<dim3(f.gbx, f.gby), f.nt_b, f.smem_b, st>>>(a);
-        else f.c<<<dim3(d->N[1], 3), f.nt_ac, f.smem_ac, st>>>(a);
-    } else {
-        size_t sac = pass_ac_smem(d), sb = pass_b_smem(d);
-        if (pass == 0) k_pass_a<<<dim3(d->N[1], 3), kPassThreads, sac, st>>>(a);
-        else if (pass == 1) k_pass_b<<<dim3((d->Hx + d->WB - 1) / d->WB, d->P[2]), kPassBThreads, sb, st>>>(a);
-        else k_pass_c<<<dim3(d->N[1], 3), kPassThreads, sac, st>>>(a);
-    }
-    UMAG_LAUNCH_CHECK();
+    for (int pass = 0; pass < 3; pass++) UMAG_TRY(launch_pass(d, ab, nb, pass, st));
     return UMAG_OK;
 }
 
@@ -846,7 +924,7 @@ int demag_exec(umag_demag* d, float* Bx, float* By, float* Bz, const float* mx, 
     a.m[0] = mx; a.m[1] = my; a.m[2] = mz;
     a.B[0] = Bx; a.B[1] = By; a.B[2] = Bz;
     a.vol = vol; a.Ms = Ms; a.Ms_mul = Ms_mul;
-    if (pass >= 0) return demag_launch_pass(d, a, ctx().stream, pass);
+    if (pass >= 0) return launch_pass(d, a, 1, pass, ctx().stream);
     UMAG_TRY(demag_launch(d, a, ctx().stream));
     // Exec completes before it returns, as the reference's does; a bulk copy
     // that timed out (a field left unwritten) is an error here, not a silent
@@ -856,7 +934,7 @@ int demag_exec(umag_demag* d, float* Bx, float* By, float* Bz, const float* mx, 
     if (cs == cudaStreamCaptureStatusNone) {
         unsigned n = 0;
         UMAG_TRY(demag_slab_timeouts(&n, ctx().stream));
-        if (n != 0) return set_error(UMAG_E_TIMEOUT, "demag pass C: %u spectrum-slab copies timed out", n);
+        if (n != 0) return set_error(UMAG_E_TIMEOUT, "demag: %u bulk copies timed out", n);
     }
     return UMAG_OK;
 }

@@ -1,25 +1,31 @@
-// demag_fast.cu -- the demag passes with compile-time FFT plans.
+// demag_fast.cu -- the fused x/z passes of common three-dimensional sizes, and
+// the choice of the pass kernels of a plan.
 //
-// Same three passes and data layout as demag.cu (see its header comment),
-// instantiated for the mesh sizes the benchmarks and common simulations use:
-// every FFT index computation is a constant, register arrays are unrolled,
-// twiddles are staged in shared memory.  demag_fast_select() returns the
-// instantiation for a plan, or nothing (the generic kernels then run).
+// Pass A: x transform, then z transform of one (y, component) slab in one
+// CTA; pass C the reverse.  Compared with separate X and Z passes
+// (demag_lines.cuh) the spectrum is written and read once less.
 #include <mutex>
+#include <set>
+#include <utility>
 
-#include "demag.cuh"
+#include "demag_inst.cuh"
 #include "fft_pair.cuh"
 #include "fft_reg.cuh"
-#include "fft_static.cuh"
 #include "tile.cuh"
 
 namespace umag {
 
-// pass C slab loads that gave up waiting (bounded mbarrier poll); the plain
-// device-op API reads it after each demag_exec (engine launches report the
-// timeout through the controller status instead, PassArgs::fault)
+// bulk copies of the passes that gave up waiting (bounded mbarrier poll); the
+// plain device-op API reads it after each demag_exec (engine launches report
+// the timeout through the controller status instead, PassArgs::fault)
 __device__ unsigned g_slab_timeouts = 0;
 
+int demag_timeouts_ptr(unsigned** out) {
+    void* p = nullptr;
+    UMAG_CUDA(cudaGetSymbolAddress(&p, g_slab_timeouts));
+    *out = static_cast<unsigned*>(p);
+    return UMAG_OK;
+}
 int demag_slab_timeouts(unsigned* out, cudaStream_t st) {
     UMAG_CUDA(cudaMemcpyFromSymbolAsync(out, g_slab_timeouts, sizeof(unsigned), 0, cudaMemcpyDeviceToHost, st));
     UMAG_CUDA(cudaStreamSynchronize(st));
@@ -31,496 +37,9 @@ int demag_set_slab_timeouts(unsigned v) {
     return UMAG_OK;
 }
 
-// record a pass that gave up waiting for a bulk copy: the counter, and the
-// instance's controller status (7, as the torque kernel's tile wait) when
-// the launch belongs to a simulation
-__device__ __forceinline__ void pass_timeout(const PassArgs& a, int ib) {
-    atomicAdd(&g_slab_timeouts, 1u);
-    if (a.fault) atomicCAS(reinterpret_cast<int*>(reinterpret_cast<char*>(a.fault) + (long)ib * a.ctl_stride), 0, 7);
-}
-
-
-static constexpr double kMu0f = 4 * 3.1415926535897932384626433 * 1e-7;  // clh/constants.clh:5
-
-constexpr int nz_of_pz(int PZ) { return PZ == 1 ? 1 : (PZ % 2 == 0 ? PZ / 2 : (PZ + 1) / 2); }
-constexpr int kNT = 256;       // passes A, C
-constexpr int kNTB = 512;      // pass B
-constexpr int kElemCap = 24;   // complex elements per thread per FFT batch
-
-template <int M, int PZ> struct AcShape {
-    static constexpr int NZ = nz_of_pz(PZ);
-    static constexpr int XP = M + 1;                                  // row pitch (holds X[0..M])
-    static constexpr int ZB = sp_divisor_le(NZ, (kElemCap * kNT) / M);  // rows per x-FFT batch
-    static constexpr int CW = PZ == 1 ? 1 : sp_divisor_le(M, (kElemCap * kNT) / PZ < 64 ? (kElemCap * kNT) / PZ : 64);
-    static constexpr size_t smem = sizeof(float2) * ((size_t)M + PZ + (M / 2 + 1) + (size_t)NZ * XP +
-                                                     (PZ > 1 ? (size_t)PZ * CW : 0));
-};
-
-// copypadmul2.cl:13-20: MU0*Ms (FP64 product rounded to float32) * vol * m
-__device__ __forceinline__ float scaled_m(const PassArgs& a, const float* __restrict__ m, int i, float msmul) {
-    float fac = a.Ms == nullptr ? msmul : __fmul_rn(msmul, __ldg(a.Ms + i));
-    float bsat = (float)(kMu0f * (double)fac);
-    float w = a.vol == nullptr ? 1.0f : __fmul_rn(1.0f, __ldg(a.vol + i));
-    return __fmul_rn(__fmul_rn(bsat, w), __ldg(m + i));
-}
-
-// Per-instance views of PassArgs for batched launches (an ensemble of
-// same-size instances, instance ib): spectrum scratch, field output, the
-// instance's controller fields (m slots, active flag) and its Ms.  With
-// ib = 0 (single-instance kernels) every offset folds away.
-__device__ __forceinline__ float2* inst_spec(const PassArgs& a, int ib) { return a.spec + (long)ib * a.spec_stride; }
-__device__ __forceinline__ float* inst_B(const PassArgs& a, int ib, int c) { return a.B[c] + (long)ib * a.b_stride; }
-__device__ __forceinline__ bool inst_inactive(const PassArgs& a, int ib) {
-    if (!a.active) return false;
-    return !*reinterpret_cast<const int*>(reinterpret_cast<const char*>(a.active) + (long)ib * a.ctl_stride);
-}
-__device__ __forceinline__ const float* inst_m(const PassArgs& a, int ib, int c) {
-    if (!a.m_ind) return a.m[c];
-    const char* slot = reinterpret_cast<const char*>(a.m_sel ? a.m_ind_w : a.m_ind) + (long)ib * a.ctl_stride;
-    return *reinterpret_cast<float* const*>(slot) + (long)c * a.ncell;
-}
-__device__ __forceinline__ float inst_msmul(const PassArgs& a, int ib) { return a.ms_mul_b ? a.ms_mul_b[ib] : a.Ms_mul; }
-
-template <int M, int PZ>
-__device__ __forceinline__ void k_fast_a_body(const PassArgs& a, const int bx, const int by, const int ib) {
-    using S = AcShape<M, PZ>;
-    constexpr int NZ = S::NZ, XP = S::XP, CW = S::CW, H = M / 2;
-    extern __shared__ __align__(16) float2 sm[];
-    float2* twx = sm;
-    float2* twz = twx + M;
-    float2* twr = twz + PZ;
-    float2* X1 = twr + (H + 1);
-    float2* Z2 = X1 + NZ * XP;
-    if (inst_inactive(a, ib)) return;
-    const int tid = threadIdx.x;
-    for (int i = tid; i < M; i += kNT) twx[i] = a.fx.tw[i];
-    if (PZ > 1)
-        for (int i = tid; i < PZ; i += kNT) twz[i] = a.fz.tw[i];
-    for (int i = tid; i <= H; i += kNT) twr[i] = a.twr[i];
-    const int y = bx, c = by, Ny = a.Ny;
-    const float* __restrict__ m = inst_m(a, ib, c);
-    const float msm = inst_msmul(a, ib);
-    // 1. scaled m, pairs of reals packed into complex (x = 2n, 2n+1), Nx = M
-    for (int e = tid; e < NZ * M; e += kNT) {
-        const int z = e / M, n = e % M;
-        float2 v = make_float2(0.f, 0.f);  // x >= Nx is zero padding
-        if (n < H) {
-            const int i = (z * Ny + y) * M + 2 * n;
-            v = make_float2(scaled_m(a, m, i, msm), scaled_m(a, m, i + 1, msm));
-        }
-        X1[z * XP + n] = v;
-    }
-    __syncthreads();
-    // 2. length-M complex FFT of every row
-#pragma unroll 1
-    for (int rb = 0; rb < NZ; rb += S::ZB) sfft<float2, M, S::ZB, kNT, XP, 1, false, -1>(X1 + rb * XP, twx);
-    // 3. R2C unpack: X[k] = E + W^k O, X[M-k] = conj(E - W^k O)
-    for (int e = tid; e < NZ * (H + 1); e += kNT) {
-        const int z = e / (H + 1), k = e % (H + 1);
-        float2* row = X1 + z * XP;
-        const int k2 = M - k;
-        float2 A = row[k], B = row[k == 0 ? 0 : k2];
-        float2 E = make_float2(0.5f * (A.x + B.x), 0.5f * (A.y - B.y));
-        float2 D = make_float2(0.5f * (A.x - B.x), 0.5f * (A.y + B.y));
-        float2 O = make_float2(D.y, -D.x);
-        float2 W = twr[k];
-        float2 WO = make_float2(W.x * O.x - W.y * O.y, W.x * O.y + W.y * O.x);
-        row[k] = make_float2(E.x + WO.x, E.y + WO.y);
-        row[k2] = make_float2(E.x - WO.x, WO.y - E.y);
-    }
-    __syncthreads();
-    float2* out = inst_spec(a, ib) + (long)c * PZ * Ny * a.Lx + (long)y * a.Lx;
-    const long kzs = (long)Ny * a.Lx;
-    if constexpr (PZ == 1) {
-        for (int k = tid; k <= M; k += kNT) out[k] = X1[k];
-    } else {
-        // 4. forward z FFT per block of CW columns, then the Nyquist column kx = M
-#pragma unroll 1
-        for (int kx0 = 0; kx0 < M; kx0 += CW) {
-            for (int e = tid; e < PZ * CW; e += kNT) {
-                const int z = e / CW, w = e % CW;
-                Z2[e] = z < NZ ? X1[z * XP + kx0 + w] : make_float2(0.f, 0.f);
-            }
-            __syncthreads();
-            sfft<float2, PZ, CW, kNT, 1, CW, true, -1>(Z2, twz);
-            for (int e = tid; e < PZ * CW; e += kNT) {
-                const int kz = e / CW, w = e % CW;
-                out[kz * kzs + kx0 + w] = Z2[e];
-            }
-            __syncthreads();
-        }
-        for (int z = tid; z < PZ; z += kNT) Z2[z] = z < NZ ? X1[z * XP + M] : make_float2(0.f, 0.f);
-        __syncthreads();
-        sfft<float2, PZ, 1, kNT, 1, 1, true, -1>(Z2, twz);
-        for (int kz = tid; kz < PZ; kz += kNT) out[kz * kzs + M] = Z2[kz];
-    }
-}
-template <int M, int PZ>
-__global__ void __launch_bounds__(kNT) k_fast_a(PassArgs a) { k_fast_a_body<M, PZ>(a, blockIdx.x, blockIdx.y, 0); }
-// batched: blockIdx.y = index + per * instance (the inst_* views above)
-template <int M, int PZ>
-__global__ void __launch_bounds__(kNT) k_fast_a_bat(PassArgs a) {
-    const int per = 3, b = blockIdx.y / per;
-    k_fast_a_body<M, PZ>(a, blockIdx.x, blockIdx.y - b * per, b);
-}
-
-template <int M, int PZ>
-__device__ __forceinline__ void k_fast_c_body(const PassArgs& a, const int bx, const int by, const int ib) {
-    using S = AcShape<M, PZ>;
-    constexpr int NZ = S::NZ, XP = S::XP, CW = S::CW, H = M / 2;
-    extern __shared__ __align__(16) float2 sm[];
-    float2* twx = sm;
-    float2* twz = twx + M;
-    float2* twr = twz + PZ;
-    float2* X1 = twr + (H + 1);
-    float2* Z2 = X1 + NZ * XP;
-    if (inst_inactive(a, ib)) return;
-    const int tid = threadIdx.x;
-    for (int i = tid; i < M; i += kNT) twx[i] = a.fx.tw[i];
-    if (PZ > 1)
-        for (int i = tid; i < PZ; i += kNT) twz[i] = a.fz.tw[i];
-    for (int i = tid; i <= H; i += kNT) twr[i] = a.twr[i];
-    const int y = bx, c = by, Ny = a.Ny;
-    const float2* in = inst_spec(a, ib) + (long)c * PZ * Ny * a.Lx + (long)y * a.Lx;
-    const long kzs = (long)Ny * a.Lx;
-    // 1. inverse z FFT per block of columns, keep z < NZ
-    if constexpr (PZ == 1) {
-        for (int k = tid; k <= M; k += kNT) X1[k] = in[k];
-    } else {
-#pragma unroll 1
-        for (int kx0 = 0; kx0 < M; kx0 += CW) {
-            for (int e = tid; e < PZ * CW; e += kNT) {
-                const int kz = e / CW, w = e % CW;
-                Z2[e] = in[kz * kzs + kx0 + w];
-            }
-            __syncthreads();
-            sfft<float2, PZ, CW, kNT, 1, CW, true, +1>(Z2, twz);
-            for (int e = tid; e < NZ * CW; e += kNT) {
-                const int z = e / CW, w = e % CW;
-                X1[z * XP + kx0 + w] = Z2[e];
-            }
-            __syncthreads();
-        }
-        for (int kz = tid; kz < PZ; kz += kNT) Z2[kz] = in[kz * kzs + M];
-        __syncthreads();
-        sfft<float2, PZ, 1, kNT, 1, 1, true, +1>(Z2, twz);
-        for (int z = tid; z < NZ; z += kNT) X1[z * XP + M] = Z2[z];
-    }
-    __syncthreads();
-    // 2. C2R pack: Z[k] = (X[k] + conj X[M-k]) + i conj(W^k) (X[k] - conj X[M-k])
-    for (int e = tid; e < NZ * (H + 1); e += kNT) {
-        const int z = e / (H + 1), k = e % (H + 1);
-        float2* row = X1 + z * XP;
-        const int k2 = M - k;
-        float2 Xk = row[k], Xm = row[k2];
-        if (k == 0) { Xk.y = 0.f; Xm.y = 0.f; }
-        float2 W = twr[k];
-        float2 S1 = make_float2(Xk.x + Xm.x, Xk.y - Xm.y);
-        float2 D1 = make_float2(Xk.x - Xm.x, Xk.y + Xm.y);
-        float2 T1 = make_float2(W.x * D1.x + W.y * D1.y, W.x * D1.y - W.y * D1.x);  // conj(W) * D1
-        float2 Zk = make_float2(S1.x - T1.y, S1.y + T1.x);
-        if (k == 0) {
-            row[0] = Zk;
-        } else {
-            float2 S2 = make_float2(Xm.x + Xk.x, Xm.y - Xk.y);
-            float2 D2 = make_float2(Xm.x - Xk.x, Xm.y + Xk.y);
-            float2 T2 = make_float2(-(W.x * D2.x - W.y * D2.y), -(W.x * D2.y + W.y * D2.x));  // -W * D2
-            row[k] = Zk;
-            row[k2] = make_float2(S2.x - T2.y, S2.y + T2.x);
-        }
-    }
-    __syncthreads();
-    // 3. inverse length-M FFT of every row
-#pragma unroll 1
-    for (int rb = 0; rb < NZ; rb += S::ZB) sfft<float2, M, S::ZB, kNT, XP, 1, false, +1>(X1 + rb * XP, twx);
-    // 4. unpack even/odd samples, crop and overwrite B (copyunpad.cl)
-    float* __restrict__ B = inst_B(a, ib, c);
-    for (int e = tid; e < NZ * H; e += kNT) {
-        const int z = e / H, n = e % H;
-        float2 v = X1[z * XP + n];
-        *reinterpret_cast<float2*>(B + (z * Ny + y) * M + 2 * n) = v;
-    }
-}
-template <int M, int PZ>
-__global__ void __launch_bounds__(kNT) k_fast_c(PassArgs a) { k_fast_c_body<M, PZ>(a, blockIdx.x, blockIdx.y, 0); }
-// batched: blockIdx.y = index + per * instance (the inst_* views above)
-template <int M, int PZ>
-__global__ void __launch_bounds__(kNT) k_fast_c_bat(PassArgs a) {
-    const int per = 3, b = blockIdx.y / per;
-    k_fast_c_body<M, PZ>(a, blockIdx.x, blockIdx.y - b * per, b);
-}
-
-template <int PY> struct BShape {
-    static constexpr int WB0 = (kElemCap * kNTB) / (3 * PY);
-    static constexpr int WB = WB0 >= 32 ? 32 : WB0 >= 16 ? 16 : WB0 >= 8 ? 8 : WB0 >= 4 ? 4 : WB0 >= 2 ? 2 : 1;
-    static constexpr size_t smem = sizeof(float2) * ((size_t)PY + (size_t)PY * 3 * WB);
-};
-
-template <int PY>
-__device__ __forceinline__ void k_fast_b_body(const PassArgs& a, const int bx, const int by, const int ib) {
-    constexpr int WB = BShape<PY>::WB, W3 = 3 * WB, NY = PY / 2, HY = PY / 2 + 1;
-    extern __shared__ __align__(16) float2 sm[];
-    float2* twy = sm;
-    float2* S = twy + PY;  // [PY][3*WB]
-    if (inst_inactive(a, ib)) return;
-    const int tid = threadIdx.x;
-    for (int i = tid; i < PY; i += kNTB) twy[i] = a.fy.tw[i];
-    const int kx0 = bx * WB, kz = by;
-    const int hx = a.Hx, Pz = a.Pz;
-    const long cs = (long)Pz * NY * a.Lx;
-    const float2* in = inst_spec(a, ib) + (long)kz * NY * a.Lx + kx0;
-    for (int e = tid; e < PY * W3; e += kNTB) {
-        const int yy = e / W3, r = e % W3, c = r / WB, w = r % WB;
-        float2 v = make_float2(0.f, 0.f);
-        if (yy < NY && kx0 + w < hx) v = in[c * cs + (long)yy * a.Lx + w];
-        S[e] = v;
-    }
-    __syncthreads();
-    sfft<float2, PY, W3, kNTB, 1, W3, true, -1>(S, twy);
-    // kernel multiply with the mirror symmetry of kernmulrsymm3d.cl:62-82
-    int kzm = kz;
-    float sz = 1.f;
-    if (kz > Pz / 2) { kzm = Pz - kz; sz = -1.f; }
-    const bool k3d = a.K[3] != nullptr;
-    for (int e = tid; e < PY * WB; e += kNTB) {
-        const int ky = e / WB, w = e % WB;
-        const int kx = kx0 + w;
-        if (kx >= hx) continue;
-        int kym = ky;
-        float sy = 1.f;
-        if (ky > NY) { kym = PY - ky; sy = -1.f; }
-        const long I = ((long)kzm * HY + kym) * a.Kp + kx;
-        const float Kxx = __ldg(a.K[0] + I), Kyy = __ldg(a.K[1] + I), Kzz = __ldg(a.K[2] + I);
-        const float Kxy = __ldg(a.K[5] + I) * sy;
-        float Kyz = 0.f, Kxz = 0.f;
-        if (k3d) {
-            Kyz = __ldg(a.K[3] + I) * (sy * sz);
-            Kxz = __ldg(a.K[4] + I) * sz;
-        }
-        float2* row = S + ky * W3;
-        const float2 mx = row[w], my = row[WB + w], mz = row[2 * WB + w];
-        row[w] = make_float2(mx.x * Kxx + my.x * Kxy + mz.x * Kxz, mx.y * Kxx + my.y * Kxy + mz.y * Kxz);
-        row[WB + w] = make_float2(mx.x * Kxy + my.x * Kyy + mz.x * Kyz, mx.y * Kxy + my.y * Kyy + mz.y * Kyz);
-        row[2 * WB + w] = make_float2(mx.x * Kxz + my.x * Kyz + mz.x * Kzz, mx.y * Kxz + my.y * Kyz + mz.y * Kzz);
-    }
-    __syncthreads();
-    sfft<float2, PY, W3, kNTB, 1, W3, true, +1>(S, twy);
-    float2* outp = inst_spec(a, ib) + (long)kz * NY * a.Lx + kx0;
-    for (int e = tid; e < NY * W3; e += kNTB) {
-        const int yy = e / W3, r = e % W3, c = r / WB, w = r % WB;
-        if (kx0 + w < hx) outp[c * cs + (long)yy * a.Lx + w] = S[e];
-    }
-}
-template <int PY>
-__global__ void __launch_bounds__(kNTB) k_fast_b(PassArgs a) { k_fast_b_body<PY>(a, blockIdx.x, blockIdx.y, 0); }
-// batched: blockIdx.y = index + per * instance (the inst_* views above)
-template <int PY>
-__global__ void __launch_bounds__(kNTB) k_fast_b_bat(PassArgs a) {
-    const int per = a.Pz, b = blockIdx.y / per;
-    k_fast_b_body<PY>(a, blockIdx.x, blockIdx.y - b * per, b);
-}
-
-// cp.async (global -> shared, asynchronous) helpers
-__device__ __forceinline__ void cpa16(void* dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
-                 "l"(src));
-}
-__device__ __forceinline__ void cpa8(void* dst, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
-                 "l"(src));
-}
-__device__ __forceinline__ void cpa4(void* dst, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
-                 "l"(src));
-}
-__device__ __forceinline__ void cpa_commit() { asm volatile("cp.async.commit_group;\n" ::); }
-__device__ __forceinline__ void cpa_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::); }
-
-// Offset of spectrum column kx within one (component, kz, y = 0) plane, and
-// the stride between rows y: blocked layout [kx/4][y][kx%4] or rows [y][kx].
-__device__ __forceinline__ long spec_col(const PassArgs& a, int kx) {
-    return a.blocked ? (long)(kx >> 2) * (a.Ny * 4) + (kx & 3) : (long)kx;
-}
-__device__ __forceinline__ long spec_rowstride(const PassArgs& a) { return a.blocked ? 4 : a.Lx; }
-// Index of kernel element (kz, ky, kx), kz/ky in the stored non-redundant block
-__device__ __forceinline__ long kern_idx(const PassArgs& a, int kz, int ky, int kx, int hy) {
-    return a.Kblocked ? (((long)kz * (a.Kp >> 2) + (kx >> 2)) * hy + ky) * 4 + (kx & 3)
-                      : ((long)kz * hy + ky) * a.Kp + kx;
-}
-
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
-                     smem_u32(dst)),
-                 "l"(src), "r"(bytes), "r"(smem_u32(bar))
-                 : "memory");
-}
-
-// Shared memory of a pass-B CTA (k_reg_b): the staged twiddle tables (TWN
-// slots, an even count so what follows stays 16-byte aligned), two exchange
-// buffers of WB padded lines, the kernel block [6][WB/KW][HY][KW] (KW = 4
-// columns per 16-byte piece, or WB when narrower).
-template <int PY, int WB> struct RegBShape {
-    static constexpr int KW = WB >= 4 ? 4 : WB;
-    static constexpr int TWN = (RgTw<PY>::size + 1) & ~1;
-    static constexpr size_t smem = sizeof(float2) * ((size_t)TWN + (size_t)2 * WB * rg_line<PY>()) +
-                                   sizeof(float) * (size_t)6 * (PY / 2 + 1) * WB;
-    // three CTAs per SM (80 registers) up to Py = 512; longer lines hold more
-    // live state per thread and keep two
-    static constexpr int minb = PY <= 512 && 3 * (smem + 1024) <= 227 * 1024 ? 3 : 2;
-};
-
-// Pass B with the register-blocked FFT (power-of-two Py): thread (t, w) holds
-// rows t + T*m (m < 8) of column kx0 + w for all three components.  Rows
-// y >= Ny are zero padding (m >= 4): the loads are skipped and the first
-// radix-8 butterfly folds them (dft8_zhalf); only rows y < Ny are computed by
-// the inverse and stored.  With the blocked layouts a warp's loads and stores
-// of one component are one contiguous run (WB = 4: 8 rows x 4 columns = 256
-// bytes).  The components exchange one at a time through two buffers
-// (rg_fft_fwd_seq), which with the kernel block fits three CTAs per SM; the
-// kernel block arrives by bulk copies (6 contiguous runs per 4 columns,
-// issued by one thread, completing on an mbarrier while the forward
-// transform runs), or by 16-byte cp.async pieces where the block is not
-// whole 4-column runs (narrow CTAs, the packed Nyquist column).
-template <int PY, int WB>
-__device__ __forceinline__ void k_reg_b_body(const PassArgs& a, const int bx, const int by, const int ib) {
-    constexpr int T = PY / 8, NT = T * WB, NY = PY / 2, HY = PY / 2 + 1;
-    constexpr int LP = rg_line<PY>();
-    constexpr int KW = RegBShape<PY, WB>::KW;
-    extern __shared__ __align__(16) float2 sm[];
-    float2* tw = sm;                                 // staged twiddles (RgTw<PY>)
-    float2* ex = tw + RegBShape<PY, WB>::TWN;        // [2][WB][LP] exchange lines
-    float* Ks = reinterpret_cast<float*>(ex + 2 * WB * LP);  // [6][WB/KW][HY][KW] kernel block
-    __shared__ __align__(8) uint64_t kbar;
-    if (inst_inactive(a, ib)) return;
-    const int tid = threadIdx.x;
-    const int w = tid % WB, t = (tid / WB) & (T - 1);  // t < T: the mask tells the compiler
-    const int hx = a.Hx, Pz = a.Pz;
-    // The last column block holds only the Nyquist column kx = Hx - 1.  When
-    // Pz is a multiple of WB its CTAs are packed: CTA by < Pz/WB handles that
-    // column for the WB planes kz = by*WB + w (the others exit), so the grid
-    // carries Pz/WB such CTAs instead of Pz mostly idle ones.
-    const bool nyq = bx * WB == hx - 1 && WB > 1 && Pz % WB == 0 && Pz >= WB;
-    if (nyq && by * WB >= Pz) return;
-    rg_tw_fill<PY>(tw, a.fy.tw, tid, NT);
-    const int kx0 = bx * WB;
-    const int kx = nyq ? hx - 1 : kx0 + w, kz = nyq ? by * WB + w : by;
-    auto kz_mirror = [&](int z) { return z > Pz / 2 ? Pz - z : z; };
-    const int kzm = kz_mirror(kz);
-    const float sz = kz > Pz / 2 ? -1.f : 1.f;
-    const bool k3d = a.K[3] != nullptr;
-    const int ncomp = k3d ? 6 : 4;
-    auto kcomp = [&](int cc) { return k3d ? cc : (cc == 3 ? 5 : cc); };  // 2D stores xx yy zz xy
-    // the kernel block: whole 4-column runs of the blocked kernel layout by
-    // bulk copies, else 16- or 4-byte asynchronous copies
-    bool bulk = false;
-    if constexpr (WB % 4 == 0) bulk = !nyq && a.Kblocked && kx0 + WB <= a.Kp;
-    if (bulk) {
-        if (tid == 0) {
-            mbar_init(&kbar, 1);
-            mbar_expect_tx(&kbar, (uint32_t)(sizeof(float) * ncomp * HY * WB));
-            for (int cc = 0; cc < ncomp; cc++)
-                for (int b4 = 0; b4 < WB / 4; b4++)
-                    bulk_g2s(Ks + kcomp(cc) * HY * WB + b4 * HY * 4, a.K[kcomp(cc)] + kern_idx(a, kzm, 0, kx0 + 4 * b4, HY),
-                             (uint32_t)(sizeof(float) * HY * 4), &kbar);
-        }
-    } else {
-        bool wide = false;
-        if constexpr (WB % 4 == 0) {
-            // 16-byte pieces of 4 columns (plan layouts: pitch padded to 4
-            // floats, pad columns zero)
-            wide = !nyq && a.Kp % 4 == 0 && kx0 + WB <= a.Kp;
-            if (wide) {
-                constexpr int CH = WB / 4;
-                for (int e = tid; e < ncomp * HY * CH; e += NT) {
-                    const int cc = e / (HY * CH), r = e % (HY * CH), ky = r / CH, ch = r % CH;
-                    cpa16(Ks + kcomp(cc) * HY * WB + ch * HY * 4 + ky * 4, a.K[kcomp(cc)] + kern_idx(a, kzm, ky, kx0 + 4 * ch, HY));
-                }
-            }
-        }
-        if (!wide) {
-            for (int e = tid; e < ncomp * HY * WB; e += NT) {
-                const int cc = e / (HY * WB), r = e % (HY * WB), ky = r / WB, ww = r % WB;
-                float* dst = Ks + kcomp(cc) * HY * WB + (ww / KW) * HY * KW + ky * KW + ww % KW;
-                const int kxw = nyq ? hx - 1 : kx0 + ww, kzw = nyq ? kz_mirror(by * WB + ww) : kzm;
-                if (kxw < hx) cpa4(dst, a.K[kcomp(cc)] + kern_idx(a, kzw, ky, kxw, HY));
-                else *dst = 0.f;
-            }
-        }
-        cpa_commit();
-    }
-    if (!k3d)  // 2D: no yz / xz components; zeros keep the multiply branch-free
-        for (int e = tid; e < 2 * HY * WB; e += NT) Ks[3 * HY * WB + e] = 0.f;
-    const bool col = kx < hx;
-    const long cs = (long)Pz * NY * a.Lx, rs = spec_rowstride(a);
-    const float2* in = inst_spec(a, ib) + (long)kz * NY * a.Lx + spec_col(a, kx);
-    float2 v[3][8];
-#pragma unroll
-    for (int c = 0; c < 3; c++)
-#pragma unroll
-        for (int m = 0; m < 8; m++) {
-            const int y = t + T * m;
-            v[c][m] = (m < 4 && col) ? in[c * cs + y * rs] : make_float2(0.f, 0.f);
-        }
-    __syncthreads();  // twiddles, barrier initialised
-    float2* exl = ex + w * LP;
-    const int exs = WB * LP;
-    rg_fft_fwd_seq<PY, 3, true>(v, t, exl, exs, tw);
-    if (bulk) {
-        for (int it = 0; !mbar_try_wait(&kbar, 0); it++) {
-            if (it == kTileWaitLimit && tid == 0) pass_timeout(a, ib);
-            if (it >= 2 * kTileWaitLimit) return;
-        }
-    } else {
-        cpa_wait_all();
-    }
-    __syncthreads();
-    // kernel multiply (kernmulrsymm3d.cl:41-90), mirrored into the stored block
-    const float* kcol = Ks + (w / KW) * HY * KW + w % KW;
-#pragma unroll
-    for (int m = 0; m < 8; m++) {
-        const int ky = t + T * m;
-        int kym = ky;
-        float sy = 1.f;
-        if (ky > NY) { kym = PY - ky; sy = -1.f; }
-        const float* kr = kcol + kym * KW;
-        const float Kxx = kr[0], Kyy = kr[HY * WB], Kzz = kr[2 * HY * WB];
-        const float Kxy = kr[5 * HY * WB] * sy;
-        const float Kyz = kr[3 * HY * WB] * (sy * sz);
-        const float Kxz = kr[4 * HY * WB] * sz;
-        const float2 mx = v[0][m], my = v[1][m], mz = v[2][m];
-        // conjugated products: the inverse is conj(FFT(conj(.))); explicit
-        // multiply-adds (fft.cuh: the same bits in every instantiation)
-        auto dot = [](float a, float ka, float b, float kb, float c, float kc) {
-            return fma_rn(c, kc, fma_rn(b, kb, mul_rn(a, ka)));
-        };
-        v[0][m] = make_float2(dot(mx.x, Kxx, my.x, Kxy, mz.x, Kxz), -dot(mx.y, Kxx, my.y, Kxy, mz.y, Kxz));
-        v[1][m] = make_float2(dot(mx.x, Kxy, my.x, Kyy, mz.x, Kyz), -dot(mx.y, Kxy, my.y, Kyy, mz.y, Kyz));
-        v[2][m] = make_float2(dot(mx.x, Kxz, my.x, Kyz, mz.x, Kzz), -dot(mx.y, Kxz, my.y, Kyz, mz.y, Kzz));
-    }
-    // (the barrier before the multiply separates the forward transform's last
-    // reads of the exchange buffers from the inverse's first writes)
-    rg_fft_fwd_seq<PY, 3, false>(v, t, exl, exs, tw);
-    if (col) {
-        float2* out = inst_spec(a, ib) + (long)kz * NY * a.Lx + spec_col(a, kx);
-#pragma unroll
-        for (int c = 0; c < 3; c++)
-#pragma unroll
-            for (int m = 0; m < 4; m++) {
-                const int y = t + T * m;
-                out[c * cs + y * rs] = make_float2(v[c][m].x, -v[c][m].y);
-            }
-    }
-}
-template <int PY, int WB>
-__global__ void __launch_bounds__((PY / 8) * WB, RegBShape<PY, WB>::minb) k_reg_b(PassArgs a) {
-    k_reg_b_body<PY, WB>(a, blockIdx.x, blockIdx.y, 0);
-}
-// batched: blockIdx.y = index + per * instance (the inst_* views above)
-template <int PY, int WB>
-__global__ void __launch_bounds__((PY / 8) * WB, RegBShape<PY, WB>::minb) k_reg_b_bat(PassArgs a) {
-    const int per = a.Pz, b = blockIdx.y / per;
-    k_reg_b_body<PY, WB>(a, blockIdx.x, blockIdx.y - b * per, b);
-}
+constexpr int nz_of_pz(int PZ) { return PZ / 2; }
+// offset of spectrum column kx within one (component, kz) plane, y = 0
+__device__ __forceinline__ long spec_col(int Ny, int kx) { return spec_at(Ny, kx, 0); }
 
 // ---- passes A and C with the register-blocked FFT (3D, power-of-two sizes)
 // x transform: TX = M/8 threads per row (one row per warp or less), rows z
@@ -615,7 +134,7 @@ __device__ __forceinline__ void k_reg_a_body(const PassArgs& a, const int bx, co
         if (k == 0) xrow[M] = make_float2(A.x - A.y, 0.f);  // Nyquist: Re Z0 - Im Z0
     }
     __syncthreads();
-    float2* out = inst_spec(a, ib) + (long)c * PZ * Ny * a.Lx + (long)y * spec_rowstride(a);
+    float2* out = inst_spec(a, ib) + (long)c * PZ * Ny * a.Lx + (long)y * 4;
     const long kzs = (long)Ny * a.Lx;
     if constexpr (PZ == 16 || PZ == 32) {
         // z phase on lane pairs, decimation in frequency: with x[n] = 0 for
@@ -631,7 +150,7 @@ __device__ __forceinline__ void k_reg_a_body(const PassArgs& a, const int bx, co
         // pair partners are lanes l and l ^ 16: a half-warp reads and writes 16
         // consecutive columns of one row
         const int t2 = (tid >> 4) & 1, cl2 = ((tid >> 5) << 4) | (tid & 15);
-        const long kM = spec_col(a, M);
+        const long kM = spec_col(Ny, M);
         // With one column per pair, the (y, component) slab of the blocked
         // spectrum is assembled in the x/z scratch ([kz][kx/4][kx%4], 128-byte
         // aligned; Xs is read into registers first) and written by one bulk
@@ -674,7 +193,7 @@ __device__ __forceinline__ void k_reg_a_body(const PassArgs& a, const int bx, co
 #pragma unroll
                 for (int r = 0; r < E2; r++) sl[((2 * r + t2) * KB + (kx >> 2)) * 4 + (kx & 3)] = u[r];
             } else {
-                const long ko = spec_col(a, kx);
+                const long ko = spec_col(Ny, kx);
 #pragma unroll
                 for (int r = 0; r < E2; r++) out[(long)(2 * r + t2) * kzs + ko] = u[r];
             }
@@ -734,12 +253,12 @@ __device__ __forceinline__ void k_reg_a_body(const PassArgs& a, const int bx, co
                     for (int j = 0; j < 8; j++) {
                         const float2 P = u[0][j], Q = pr[j];
                         out[(tz + TZ * j) * kzs] = make_float2(0.5f * (P.x + Q.x), 0.5f * (P.y - Q.y));
-                        out[(tz + TZ * j) * kzs + spec_col(a, M)] = make_float2(0.5f * (P.y + Q.y), -0.5f * (P.x - Q.x));
+                        out[(tz + TZ * j) * kzs + spec_col(Ny, M)] = make_float2(0.5f * (P.y + Q.y), -0.5f * (P.x - Q.x));
                     }
                     continue;
                 }
             }
-            const long ko = spec_col(a, kx);
+            const long ko = spec_col(Ny, kx);
     #pragma unroll
             for (int j = 0; j < 8; j++) out[(tz + TZ * j) * kzs + ko] = u[0][j];
         }
@@ -797,7 +316,7 @@ __device__ __forceinline__ void k_reg_c_body(const PassArgs& a, const int bx, co
             if (it >= 2 * kTileWaitLimit) return;
         }
     }
-    const float2* in = inst_spec(a, ib) + (long)c * PZ * Ny * a.Lx + (long)y * spec_rowstride(a);
+    const float2* in = inst_spec(a, ib) + (long)c * PZ * Ny * a.Lx + (long)y * 4;
     const long kzs = (long)Ny * a.Lx;
     if constexpr (PZ == 16 || PZ == 32) {
         // z phase on lane pairs, inverse by the conjugate trick, decimation in
@@ -813,12 +332,12 @@ __device__ __forceinline__ void k_reg_c_body(const PassArgs& a, const int bx, co
         // consecutive columns of one row (conflict-free in shared memory)
         static_assert(NT % 32 == 0, "whole warps of lane pairs");
         const int t2 = (tid >> 4) & 1, cl2 = ((tid >> 5) << 4) | (tid & 15);
-        const long kM = spec_col(a, M);
+        const long kM = spec_col(Ny, M);
 #pragma unroll
         for (int r0 = 0; r0 < M / CP2; r0++) {
             const int kx = r0 * CP2 + cl2;
             const bool pk = kx == 0;
-            const long ko = spec_col(a, kx);
+            const long ko = spec_col(Ny, kx);
             float2 u[E2];
 #pragma unroll
             for (int j = 0; j < E2; j++) {
@@ -866,7 +385,7 @@ __device__ __forceinline__ void k_reg_c_body(const PassArgs& a, const int bx, co
         float2 u[2][1][8];
     #pragma unroll
         for (int r = 0; r < 2; r++) {
-            const long ko = spec_col(a, r * CPR + cl), kM = spec_col(a, M);
+            const long ko = spec_col(Ny, r * CPR + cl), kM = spec_col(Ny, M);
     #pragma unroll
             for (int j = 0; j < 8; j++) {
                 float2 q = in[(tz + TZ * j) * kzs + ko];
@@ -931,165 +450,96 @@ __global__ void __launch_bounds__(RegAC<M, PZ>::NT) k_reg_c_bat(PassArgs a) {
     k_reg_c_body<M, PZ>(a, blockIdx.x, blockIdx.y - b * per, b);
 }
 
-template <int PY> struct RegB {
-    static constexpr int T = PY / 8;
-    static constexpr int WB = T >= 256 ? 1 : 256 / T > 16 ? 16 : 256 / T;
-    static constexpr int NT = T * WB;
-    static constexpr size_t smem = RegBShape<PY, WB>::smem;
-};
-
-// one warp per CTA (or one column): for small meshes, where the default
-// shape leaves most SMs idle
-template <int PY> struct RegBNarrow {
-    static constexpr int T = PY / 8;
-    static constexpr int WB = T >= 32 ? 1 : 32 / T;
-    static constexpr int NT = T * WB;
-    static constexpr size_t smem = RegBShape<PY, WB>::smem;
-};
-
-// ------------------------------------------------------------------ dispatch
-template <int M, int PZ> static void fill_ac(FastPasses& f) {
-    if constexpr (RegAC<M, PZ>::ok && PZ >= 8) {
-        f.a = k_reg_a<M, PZ>;
-        f.c = k_reg_c<M, PZ>;
-        f.ab = k_reg_a_bat<M, PZ>;
-        f.cb = k_reg_c_bat<M, PZ>;
-        f.smem_ac = RegAC<M, PZ>::smem;
-        f.ac_scratch = sizeof(float2) * ((size_t)RegAC<M, PZ>::NZ * RegAC<M, PZ>::XP + RegAC<M, PZ>::EXN);
-        f.slab_ok = (PZ == 16 || PZ == 32) && M / (RegAC<M, PZ>::NT / 2) == 1;
-        f.nt_ac = RegAC<M, PZ>::NT;
-        f.ac_reg = true;
-    } else {
-        f.a = k_fast_a<M, PZ>;
-        f.c = k_fast_c<M, PZ>;
-        f.ab = k_fast_a_bat<M, PZ>;
-        f.cb = k_fast_c_bat<M, PZ>;
-        f.smem_ac = AcShape<M, PZ>::smem;
-        f.nt_ac = kNT;
-    }
+// ------------------------------------------------------------------ choice of kernels
+template <int M, int PZ> static void fill_fused(Passes& f) {
+    using S = RegAC<M, PZ>;
+    static_assert(S::ok, "register x/z passes");
+    f.a = k_reg_a<M, PZ>;
+    f.c = k_reg_c<M, PZ>;
+    f.ab = k_reg_a_bat<M, PZ>;
+    f.cb = k_reg_c_bat<M, PZ>;
+    f.smem_ac = S::smem;
+    f.ac_scratch = sizeof(float2) * ((size_t)S::NZ * S::XP + S::EXN);
+    f.slab_ok = (PZ == 16 || PZ == 32) && M / (S::NT / 2) == 1;
+    f.nt_ac = S::NT;
 }
-template <int PY> static void fill_b(FastPasses& f) {
-    if constexpr (rg_ok(PY) && PY >= 32) {
-        f.b = k_reg_b<PY, RegB<PY>::WB>;
-        f.bb = k_reg_b_bat<PY, RegB<PY>::WB>;
-        f.smem_b = RegB<PY>::smem;
-        f.wb = RegB<PY>::WB;
-        f.nt_b = RegB<PY>::NT;
-        f.b_reg = true;
-        if constexpr (RegBNarrow<PY>::WB < RegB<PY>::WB) {
-            f.b_n = k_reg_b<PY, RegBNarrow<PY>::WB>;
-            f.smem_b_n = RegBNarrow<PY>::smem;
-            f.wb_n = RegBNarrow<PY>::WB;
-            f.nt_b_n = RegBNarrow<PY>::NT;
-        }
-    } else {
-        f.b = k_fast_b<PY>;
-        f.bb = k_fast_b_bat<PY>;
-        f.smem_b = BShape<PY>::smem;
-        f.wb = BShape<PY>::WB;
-        f.nt_b = kNTB;
-    }
-}
-
-bool demag_fast_select(int M, int Py, int Pz, FastPasses& f) {
-    f = FastPasses{};
-    bool ac = true;
-#define AC(m, pz) else if (M == m && Pz == pz) fill_ac<m, pz>(f);
-    if (false) {}
-    AC(16, 1) AC(24, 1) AC(32, 1) AC(48, 1) AC(64, 1) AC(96, 1) AC(128, 1) AC(192, 1) AC(256, 1) AC(384, 1)
-    AC(512, 1) AC(1024, 1)
-    AC(64, 12) AC(64, 16) AC(64, 32) AC(64, 64)
-    AC(128, 12) AC(128, 16) AC(128, 32) AC(128, 64)
-    AC(256, 12) AC(256, 16) AC(256, 32) AC(256, 64)
-    AC(512, 12) AC(512, 16) AC(512, 32) AC(512, 64)
-    else ac = false;
+// meshes of exactly M x (any) x PZ/2 cells
+bool fused_select(int M, int Pz, Passes& f) {
+#define AC(m, pz) if (M == m && Pz == pz) { fill_fused<m, pz>(f); return true; }
+    AC(64, 16) AC(64, 32) AC(64, 64)
+    AC(128, 16) AC(128, 32) AC(128, 64)
+    AC(256, 16) AC(256, 32) AC(256, 64)
 #undef AC
-    bool b = true;
-#define BB(py) else if (Py == py) fill_b<py>(f);
-    if (false) {}
-    BB(32) BB(48) BB(64) BB(96) BB(128) BB(192) BB(256) BB(384) BB(512) BB(1024) BB(2048)
-    else b = false;
-#undef BB
-    if (!(ac && b)) f = FastPasses{};
-    // 4-column-block spectrum layout when all three passes are register kernels
-    f.blocked = ac && b && f.ac_reg && f.b_reg;
-    return ac && b;
+    return false;
 }
 
-int demag_fast_grid(FastPasses& f, int M, int Pz, int sm_count) {
-    if (sm_count <= 0) sm_count = ctx().sm_count;
-    f.gbx = (unsigned)((M + 1 + f.wb - 1) / f.wb);
-    f.gby = (unsigned)Pz;
-    // a default pass-B grid smaller than the SM count runs on a few SMs: such
-    // plans use CTAs of one warp instead for a single mesh (batched launches
-    // have CTAs enough and keep the default); the arithmetic per column is
-    // the same, bit for bit, because the butterflies and the kernel multiply
-    // spell out their rounding (fft.cuh)
-    if (f.b_n) {
-        f.gbx_n = (unsigned)((M + 1 + f.wb_n - 1) / f.wb_n);
-        f.use_narrow = (long)f.gbx * f.gby < sm_count;
+bool listed_mesh(const int N[3], const int P[3]) {
+    static const int m2[] = {16, 24, 32, 48, 64, 96, 128, 192, 256, 384, 512, 1024}, m3[] = {64, 128, 256, 512};
+    static const int pz3[] = {12, 16, 32, 64}, py[] = {32, 48, 64, 96, 128, 192, 256, 384, 512, 1024, 2048};
+    auto in = [](int v, const int* l, int n) {
+        for (int i = 0; i < n; i++)
+            if (l[i] == v) return true;
+        return false;
+    };
+    const bool x = P[2] == 1 ? in(N[0], m2, 12) : in(N[0], m3, 4) && in(P[2], pz3, 4);
+    return P[0] == 2 * N[0] && x && in(P[1], py, 11);
+}
+
+bool lines_select(const int N[3], const int pbc[3], int F[3], Passes& f, bool exact) {
+    f = Passes{};
+    static const int lens[] = {2, 3, 4, 5, 6, 8, 10, 12, 16, 20, 24, 30, 32, 40, 48, 50, 60, 64, 80, 96, 100, 120, 128,
+                               160, 192, 200, 256, 320, 384, 512, 640, 768, 1024};
+    auto fits = [&](int need, bool periodic, int unit, auto pick) -> int {
+        for (int l : lens) {
+            const int have = unit * l;
+            if (periodic || exact ? have == need : have >= need)
+                if (pick(l)) return have;
+        }
+        return 0;
+    };
+    // x: packed pairs of reals, half a padded line of length M per parity
+    const int py = pbc[1] ? 1 : 2, pz = pbc[2] ? 1 : 2;
+    const int M = pbc[0] ? fits(N[0] / 2, true, 1, [&](int l) { return lines_x(l, 1, f); })
+                         : fits(N[0], false, 2, [&](int l) { return lines_x(l, 2, f); });
+    const int ly = fits(N[1], pbc[1] != 0, 1, [&](int l) { return lines_y(l, py, f); });
+    if (M == 0 || ly == 0) return false;
+    F[0] = 2 * M;
+    F[1] = py * ly;
+    F[2] = 1;
+    if (N[2] > 1) {
+        const int h = fits(N[2], pbc[2] != 0, 1, [&](int l) { return lines_z(l, pz, f); });
+        if (h == 0) return false;
+        F[2] = pz * h;
+        // the fused passes transform open meshes of exactly their size
+        if (!pbc[0] && !pbc[2] && M == N[0] && 2 * N[2] == F[2]) fused_select(M, F[2], f);
     }
-    return UMAG_OK;
+    return true;
 }
 
-static int demag_fast_setup_device();
-
-int demag_fast_setup() {
+int pass_attrs(void (*k)(PassArgs)) {
     // cudaFuncSetAttribute applies to the current device's context, so the
-    // opt-in is made once per device, under a lock (host threads may race)
+    // opt-in is made once per device, under a lock (host threads may race):
+    // the full 227 KB, and the largest shared-memory carveout, so that several
+    // CTAs of these kernels fit on one SM
     static std::mutex mu;
-    static bool done[64] = {};
+    static std::set<std::pair<int, const void*>> done;
+    if (!k) return UMAG_OK;
     int dev = 0;
     UMAG_CUDA(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 64) return set_error(UMAG_E_ARG, "device %d out of range", dev);
     std::lock_guard<std::mutex> lock(mu);
-    if (done[dev]) return UMAG_OK;
-    UMAG_TRY(demag_fast_setup_device());
-    done[dev] = true;
+    const std::pair<int, const void*> key{dev, reinterpret_cast<const void*>(k)};
+    if (done.count(key)) return UMAG_OK;
+    cudaFuncAttributes fa;  // the opt-in covers static + dynamic shared memory
+    UMAG_CUDA(cudaFuncGetAttributes(&fa, k));
+    UMAG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   227 * 1024 - (int)fa.sharedSizeBytes));
+    UMAG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+    done.insert(key);
     return UMAG_OK;
 }
 
-static int demag_fast_setup_device() {
-    // opt in to the full 227 KB and ask for the largest shared-memory carveout,
-    // so several CTAs of these shared-memory-heavy kernels fit on one SM
-    auto attrs = [](void (*k)(PassArgs)) -> int {
-        cudaFuncAttributes fa;  // the opt-in covers static + dynamic shared memory
-        UMAG_CUDA(cudaFuncGetAttributes(&fa, k));
-        UMAG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       227 * 1024 - (int)fa.sharedSizeBytes));
-        UMAG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                       cudaSharedmemCarveoutMaxShared));
-        return UMAG_OK;
-    };
-    FastPasses f;
-    const int Ms[] = {16, 24, 32, 48, 64, 96, 128, 192, 256, 384, 512, 1024};
-    for (int m : Ms)
-        if (demag_fast_select(m, 2 * m > 2048 ? 2048 : 2 * m, 1, f)) {
-            UMAG_TRY(attrs(f.a));
-            UMAG_TRY(attrs(f.c));
-            UMAG_TRY(attrs(f.ab));
-            UMAG_TRY(attrs(f.cb));
-        }
-    const int m3[] = {64, 128, 256, 512}, pz3[] = {12, 16, 32, 64};
-    for (int m : m3)
-        for (int pz : pz3)
-            if (demag_fast_select(m, 2 * m, pz, f)) {
-                UMAG_TRY(attrs(f.a));
-                UMAG_TRY(attrs(f.c));
-                UMAG_TRY(attrs(f.ab));
-                UMAG_TRY(attrs(f.cb));
-            }
-    // pass B instantiations
-    {
-        FastPasses g{};
-#define SETB(py)                                     \
-    fill_b<py>(g);                                   \
-    UMAG_TRY(attrs(g.b));                            \
-    UMAG_TRY(attrs(g.bb));                           \
-    if (g.b_n) UMAG_TRY(attrs(g.b_n));
-        SETB(32) SETB(48) SETB(64) SETB(96) SETB(128) SETB(192) SETB(256) SETB(384) SETB(512) SETB(1024) SETB(2048)
-#undef SETB
-    }
+int passes_attrs(const Passes& f) {
+    for (auto k : {f.xf, f.xi, f.zf, f.zi, f.y, f.a, f.c, f.ab, f.cb}) UMAG_TRY(pass_attrs(k));
     return UMAG_OK;
 }
 

@@ -805,7 +805,7 @@ static int launch_torque(SimImpl* s, int m_sel, int slot, float* tau_direct, flo
         a.m_sel = m_sel;
         if (s->batched) UMAG_TRY(demag_launch_batch(s->demag, a, s->nb, S()));
         else UMAG_TRY(demag_launch(s->demag, a, S()));
-        if (nl) *nl += 3;
+        if (nl) *nl += demag_launches(s->demag);
     }
     LocalArgs la = s->la;
     la.m_sel = m_sel;
@@ -1941,7 +1941,7 @@ static int ens_class_new(EnsClass& C, const umag_ens_instance* in, const std::ve
     UMAG_CUDA(cudaStreamSynchronize(S()));
     if (demag) {
         fill_pass_args(s->demag, s->pa);
-        const long spec_elems = 3L * s->demag->P[2] * s->demag->N[1] * s->demag->Lx;  // one plan's spectrum
+        const long spec_elems = 3L * s->demag->F[2] * s->demag->N[1] * s->demag->Lx;  // one plan's spectrum
         UMAG_CUDA(cudaMalloc(&C.spec, sizeof(float2) * spec_elems * nb));
         UMAG_CUDA(cudaMemsetAsync(C.spec, 0, sizeof(float2) * spec_elems * nb, S()));
         s->pa.spec = C.spec;

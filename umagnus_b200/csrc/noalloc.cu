@@ -100,15 +100,11 @@ extern "C" __attribute__((visibility("default"))) int umag_demag_exec_noalloc(
     d.Lx = (d.Hx + 3) / 4 * 4;
     d.is2d = Nz == 1;
     if (Nz > 1) UMAG_REQUIRE(K[3] && K[4], "NULL yz/xz kernel spectrum for a 3D mesh");
-    UMAG_TRY(demag_fast_setup());
-    if (!demag_fast_select(d.M, d.P[1], d.P[2], d.fast))
+    const int pbc[3] = {0, 0, 0};
+    if (!listed_mesh(d.N, d.P) || !lines_select(d.N, pbc, d.F, d.fast, true) || d.F[2] != d.P[2])
         return set_error(UMAG_E_UNSUPPORTED, "mesh %dx%dx%d has no compile-time FFT plan (no-alloc path)", Nx, Ny, Nz);
-    int dev = 0, sms = 0;
-    UMAG_CUDA(cudaGetDevice(&dev));
-    UMAG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    UMAG_TRY(demag_fast_grid(d.fast, d.M, d.P[2], sms));
-    d.use_fast = true;
-    d.WB = d.fast.wb;
+    UMAG_TRY(passes_attrs(d.fast));
+    d.use_lines = true;
     // scratch layout: spectrum | tw(M) | tw(Py) | tw(Pz) | exp(-2 pi i k/Px), k < M
     const size_t spec = (size_t)3 * d.P[2] * Ny * d.Lx;
     const size_t ntw = (size_t)d.M + d.P[1] + d.P[2] + d.M;
@@ -130,14 +126,14 @@ extern "C" __attribute__((visibility("default"))) int umag_demag_exec_noalloc(
     PassArgs a{};
     a.Nx = Nx; a.Ny = Ny; a.Nz = Nz;
     a.Px = d.P[0]; a.Py = d.P[1]; a.Pz = d.P[2];
-    a.M = d.M; a.Hx = d.Hx; a.HxP = d.HxP; a.Lx = d.Lx; a.WB = d.WB;
+    a.M = d.M; a.Hx = d.Hx; a.HxP = d.HxP; a.Lx = d.Lx;
     a.fx = fx; a.fy = fy; a.fz = fz;
     a.twr = tw + d.M + d.P[1] + d.P[2];
     a.spec = sp;
     for (int c = 0; c < 6; c++) a.K[c] = K[c];
     a.Kp = d.Hx;  // caller's spectrum: reference layout, rows of Px/2+1 floats
     a.Kblocked = 0;
-    a.blocked = d.fast.blocked ? 1 : 0;
+    UMAG_TRY(demag_timeouts_ptr(&a.timeouts));
     if (d.is2d) a.K[3] = a.K[4] = nullptr;
     a.m[0] = mx; a.m[1] = my; a.m[2] = mz;
     a.B[0] = Bx; a.B[1] = By; a.B[2] = Bz;
