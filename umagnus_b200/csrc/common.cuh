@@ -5,6 +5,7 @@
 #include <cstdarg>
 #include <cstdint>
 #include <cstdio>
+#include <utility>
 
 #include "../../include/umagnus_b200.h"
 
@@ -56,6 +57,32 @@ inline int grid_for(long long n, int block, int waves = 8) {
     long long cap = (long long)ctx().sm_count * waves;
     if (need < 1) need = 1;
     return (int)(need < cap ? need : cap);
+}
+
+// Programmatic dependent launch.  A kernel queued with launch_pdl may start
+// while the kernel before it in the stream (or graph) still runs: its CTAs are
+// placed as that kernel's last CTAs leave, and set themselves up (tables,
+// barriers) until pdl_wait.  After pdl_wait every earlier kernel is complete
+// and its writes are visible.  Every CTA of a kernel calls pdl_wait, then
+// pdl_trigger, before it returns; so what precedes pdl_wait may read what the
+// kernels before the last one wrote (that last one had itself waited before
+// it let this one start).  Queued any other way, the calls do nothing.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+template <class... P, class... A>
+inline cudaError_t launch_pdl(bool overlap, void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                              A&&... args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = overlap ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, k, std::forward<A>(args)...);
 }
 
 }  // namespace umag

@@ -859,7 +859,8 @@ void fill_pass_args(const umag_demag* d, PassArgs& a) {
 
 // pass 0: scaled m to the spectrum (x, z), 1: y and the kernel, 2: back to B,
 // for nb instances at once
-static int launch_pass(const umag_demag* d, const PassArgs& a, int nb, int pass, cudaStream_t st) {
+// ov: overlap with the kernel before (launch_pdl)
+static int launch_pass(const umag_demag* d, const PassArgs& a, int nb, int pass, cudaStream_t st, bool ov) {
     const int Nx3 = 3 * d->N[2], Ny = d->N[1];
     if (!d->use_lines) {
         const size_t sac = pass_ac_smem(d), sb = pass_b_smem(d);
@@ -871,28 +872,25 @@ static int launch_pass(const umag_demag* d, const PassArgs& a, int nb, int pass,
     }
     const Passes& f = d->fast;
     if (pass == 1) {
-        f.y<<<dim3(d->Lx / 4, d->F[2], nb), f.nt_y, d->is2d ? f.smem_y2 : f.smem_y3, st>>>(a);
+        UMAG_CUDA(launch_pdl(ov, f.y, dim3(d->Lx / 4, d->F[2], nb), f.nt_y, d->is2d ? f.smem_y2 : f.smem_y3, st, a));
     } else if (f.a) {
-        if (pass == 0) (nb > 1 ? f.ab : f.a)<<<dim3(Ny, 3 * nb), f.nt_ac, f.smem_ac, st>>>(a);
-        else (nb > 1 ? f.cb : f.c)<<<dim3(Ny, 3 * nb), f.nt_ac, f.smem_ac, st>>>(a);
+        auto k = pass == 0 ? (nb > 1 ? f.ab : f.a) : (nb > 1 ? f.cb : f.c);
+        UMAG_CUDA(launch_pdl(ov, k, dim3(Ny, 3 * nb), f.nt_ac, f.smem_ac, st, a));
     } else {
         const dim3 gx((Ny + 3) / 4, Nx3, nb), gz((unsigned)(((long)Ny * d->Lx + 127) / 128), 3, nb);
         if (pass == 0) {
-            f.xf<<<gx, f.nt_x, f.smem_x, st>>>(a);
-            UMAG_LAUNCH_CHECK();
-            if (f.zf) f.zf<<<gz, 128, 0, st>>>(a);
+            UMAG_CUDA(launch_pdl(ov, f.xf, gx, f.nt_x, f.smem_x, st, a));
+            if (f.zf) UMAG_CUDA(launch_pdl(ov, f.zf, gz, 128, 0, st, a));
         } else {
-            if (f.zi) f.zi<<<gz, 128, 0, st>>>(a);
-            UMAG_LAUNCH_CHECK();
-            f.xi<<<gx, f.nt_x, f.smem_x, st>>>(a);
+            if (f.zi) UMAG_CUDA(launch_pdl(ov, f.zi, gz, 128, 0, st, a));
+            UMAG_CUDA(launch_pdl(ov, f.xi, gx, f.nt_x, f.smem_x, st, a));
         }
     }
-    UMAG_LAUNCH_CHECK();
     return UMAG_OK;
 }
 
-int demag_launch(const umag_demag* d, const PassArgs& a, cudaStream_t st) {
-    for (int pass = 0; pass < 3; pass++) UMAG_TRY(launch_pass(d, a, 1, pass, st));
+int demag_launch(const umag_demag* d, const PassArgs& a, cudaStream_t st, bool overlap) {
+    for (int pass = 0; pass < 3; pass++) UMAG_TRY(launch_pass(d, a, 1, pass, st, pass > 0 || overlap));
     return UMAG_OK;
 }
 
@@ -904,13 +902,13 @@ int demag_launches(const umag_demag* d) {
 
 // the passes for nb same-size instances at once (the per-instance pointers
 // are shifted by the strides in PassArgs)
-int demag_launch_batch(const umag_demag* d, const PassArgs& a, int nb, cudaStream_t st) {
+int demag_launch_batch(const umag_demag* d, const PassArgs& a, int nb, cudaStream_t st, bool overlap) {
     UMAG_REQUIRE(d->use_lines && listed_mesh(d->N, d->P), "batched demag needs a compile-time FFT plan");
     UMAG_REQUIRE(nb >= 1 && 3L * nb <= 65535 && (long)d->F[2] * nb <= 65535, "too many instances in one batch");
     // per-instance spectra: the slab map covers the plan's own spectrum only
     PassArgs ab = a;
     ab.slab_map = nullptr;
-    for (int pass = 0; pass < 3; pass++) UMAG_TRY(launch_pass(d, ab, nb, pass, st));
+    for (int pass = 0; pass < 3; pass++) UMAG_TRY(launch_pass(d, ab, nb, pass, st, overlap));
     return UMAG_OK;
 }
 
@@ -924,7 +922,7 @@ int demag_exec(umag_demag* d, float* Bx, float* By, float* Bz, const float* mx, 
     a.m[0] = mx; a.m[1] = my; a.m[2] = mz;
     a.B[0] = Bx; a.B[1] = By; a.B[2] = Bz;
     a.vol = vol; a.Ms = Ms; a.Ms_mul = Ms_mul;
-    if (pass >= 0) return launch_pass(d, a, 1, pass, ctx().stream);
+    if (pass >= 0) return launch_pass(d, a, 1, pass, ctx().stream, false);
     UMAG_TRY(demag_launch(d, a, ctx().stream));
     // Exec completes before it returns, as the reference's does; a bulk copy
     // that timed out (a field left unwritten) is an error here, not a silent

@@ -120,10 +120,11 @@ int demag_get_kernel(umag_demag* d, double* const host[6]);
 int demag_get_spectrum(umag_demag* d, float* const host[6]);
 void demag_free(umag_demag* d);
 void fill_pass_args(const umag_demag* d, PassArgs& a);
-int demag_launch(const umag_demag* d, const PassArgs& a, cudaStream_t st);
+// overlap: the kernel queued before it calls pdl_wait (common.cuh)
+int demag_launch(const umag_demag* d, const PassArgs& a, cudaStream_t st, bool overlap = false);
 // kernels that demag_launch queues
 int demag_launches(const umag_demag* d);
-int demag_launch_batch(const umag_demag* d, const PassArgs& a, int nb, cudaStream_t st);
+int demag_launch_batch(const umag_demag* d, const PassArgs& a, int nb, cudaStream_t st, bool overlap = false);
 // the line kernels for mesh N and their sizes F (with the fused x/z passes of F;
 // exact: of the reference's padded sizes only); false: no such lengths
 bool lines_select(const int N[3], const int pbc[3], int F[3], Passes& f, bool exact);

@@ -68,10 +68,12 @@ __device__ __forceinline__ void k_reg_a_body(const PassArgs& a, const int bx, co
     float2* twr = twz + S::TWZ;   // M: exp(-2 pi i k / Px)
     float2* Xs = twr + M;         // [NZ][XP]
     float2* ex = Xs + NZ * XP; // exchange lines
+    pdl_wait();
+    pdl_trigger();
     if (inst_inactive(a, ib)) return;
     const int tid = threadIdx.x;
     const int y = bx, c = by, Ny = a.Ny;
-    const float* __restrict__ mp = inst_m(a, ib, c);
+    const float* mp = inst_m(a, ib, c);
     const float msm = inst_msmul(a, ib);
     // x phase: row z, lane t holds packed z[n] = x[2n] + i x[2n+1], n = t + TX*j
     const int z = tid / TX, t = tid % TX;
@@ -283,6 +285,8 @@ __device__ __forceinline__ void k_reg_c_body(const PassArgs& a, const int bx, co
     float2* twr = twz + S::TWZ;
     float2* Xs = twr + M;
     float2* ex = Xs + NZ * XP;
+    pdl_wait();
+    pdl_trigger();
     if (inst_inactive(a, ib)) return;
     const int tid = threadIdx.x;
     // the (y, component) slab of the spectrum by one bulk tensor copy into

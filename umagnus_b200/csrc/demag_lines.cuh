@@ -23,8 +23,10 @@ namespace umag {
 // row pitch or line stride of at least n slots, = r (mod 16)
 constexpr int pitch16(int n, int r) { return n + ((r - n) % 16 + 16) % 16; }
 
+// asynchronous (the loads that follow do not wait for it): cpa_wait_all and a
+// barrier come before its use
 __device__ __forceinline__ void tw_copy(float2* dst, const float2* __restrict__ src, int n, int tid, int nth) {
-    for (int i = tid; i < n; i += nth) dst[i] = __ldg(src + i);
+    for (int i = tid; i < n; i += nth) cpa8(dst + i, src + i);
 }
 
 // ================================================================ X
@@ -56,8 +58,15 @@ __global__ void __launch_bounds__(4 * NPAR * Line<L>::T) k_x_fwd(const __grid_co
     const int ib = blockIdx.z;
     const int tid = threadIdx.x, p = tid % NPAR, t = (tid / NPAR) % T, row = tid / (NPAR * T);
     const int c = blockIdx.y / a.Nz, z = blockIdx.y - c * a.Nz, y0 = blockIdx.x * 4, y = y0 + row, Nx = a.Nx;
-    const float* __restrict__ m = inst_m(a, ib, c);  // (both reads in flight before the first wait)
-    if (inst_inactive(a, ib)) return;
+    tw_copy(tw, a.fx.tw, M, tid, NT);
+    tw_copy(twr, a.twr, S::WR, tid, NT);
+    pdl_wait();
+    pdl_trigger();
+    const float* m = inst_m(a, ib, c);  // (both reads in flight before the first use)
+    if (inst_inactive(a, ib)) {
+        cpa_wait_all();
+        return;
+    }
     const float msm = inst_msmul(a, ib);
     P2 v[1][LN::NE];
     {
@@ -111,8 +120,7 @@ __global__ void __launch_bounds__(4 * NPAR * Line<L>::T) k_x_fwd(const __grid_co
             v[0][i] = p2(in && x < Nx ? f[i].x : 0.f, in && x + 1 < Nx ? f[i].y : 0.f);
         }
     }
-    tw_copy(tw, a.fx.tw, M, tid, NT);  // while the rows are in flight
-    tw_copy(twr, a.twr, S::WR, tid, NT);
+    cpa_wait_all();
     __syncthreads();
     line_fwd<LN, NPAR, 1, 1>(v, t, p, ex + row * S::SR + p * S::SP, 0, tw);
 #pragma unroll
@@ -150,9 +158,16 @@ __global__ void __launch_bounds__(4 * NPAR * Line<L>::T) k_x_inv(const __grid_co
     extern __shared__ __align__(16) float2 sm[];
     float2 *tw = sm, *twr = tw + M, *ex = twr + S::WR, *Zs = ex + 4 * S::SR;
     const int ib = blockIdx.z;
-    if (inst_inactive(a, ib)) return;
     const int tid = threadIdx.x, p = tid % NPAR, t = (tid / NPAR) % T, row = tid / (NPAR * T);
     const int c = blockIdx.y / a.Nz, z = blockIdx.y - c * a.Nz, y0 = blockIdx.x * 4, y = y0 + row, Nx = a.Nx;
+    tw_copy(tw, a.fx.tw, M, tid, NT);
+    tw_copy(twr, a.twr, S::WR, tid, NT);
+    pdl_wait();
+    pdl_trigger();
+    if (inst_inactive(a, ib)) {
+        cpa_wait_all();
+        return;
+    }
     const float2* in = inst_spec(a, ib) + ((long)c * a.Pz + z) * a.Ny * a.Lx;
     // the thread's columns k and M - k, all loads before the first use
     constexpr int NK = cdiv((M / 8 + 1) * 16, NT);
@@ -164,8 +179,7 @@ __global__ void __launch_bounds__(4 * NPAR * Line<L>::T) k_x_inv(const __grid_co
         Xk[i] = in_ ? in[spec_at(a.Ny, k, y0 + r)] : make_float2(0.f, 0.f);
         Xm[i] = in_ ? in[spec_at(a.Ny, M - k, y0 + r)] : make_float2(0.f, 0.f);
     }
-    tw_copy(tw, a.fx.tw, M, tid, NT);
-    tw_copy(twr, a.twr, S::WR, tid, NT);
+    cpa_wait_all();
     __syncthreads();
 #pragma unroll
     for (int i = 0; i < NK; i++) {
@@ -231,6 +245,8 @@ template <int H, int N = 1> __device__ __forceinline__ void z_ramp(P2 (&u)[H]) {
 // 125 us inverse for the 605 MB (5.3 and 4.8 TB/s).
 template <int H, int NPAR> __global__ void __launch_bounds__(128) k_z_fwd(const __grid_constant__ PassArgs a) {
     const int ib = blockIdx.z;
+    pdl_wait();
+    pdl_trigger();
     if (inst_inactive(a, ib)) return;
     const long ps = (long)a.Ny * a.Lx, e = blockIdx.x * 128L + threadIdx.x;
     if (e >= ps) return;
@@ -256,6 +272,8 @@ template <int H, int NPAR> __global__ void __launch_bounds__(128) k_z_fwd(const 
 }
 template <int H, int NPAR> __global__ void __launch_bounds__(128) k_z_inv(const __grid_constant__ PassArgs a) {
     const int ib = blockIdx.z;
+    pdl_wait();
+    pdl_trigger();
     if (inst_inactive(a, ib)) return;
     const long ps = (long)a.Ny * a.Lx, e = blockIdx.x * 128L + threadIdx.x;
     if (e >= ps) return;
@@ -328,7 +346,6 @@ __global__ void __launch_bounds__(4 * NPAR * Line<L>::T, YShape<L, NPAR>::minb) 
     float* Ks = reinterpret_cast<float*>(ex + S::NBUF * S::lines * S::LS);  // [comp][ky][4]
     __shared__ __align__(8) uint64_t kbar;
     const int ib = blockIdx.z;
-    if (inst_inactive(a, ib)) return;
     const int tid = threadIdx.x, w = tid & 3, p = (tid >> 2) & (NPAR - 1), t = tid / (4 * NPAR);
     const int kz = blockIdx.y, kx0 = blockIdx.x * 4, Ny = a.Ny, Pz = a.Pz;
     const int kzm = kz > Pz / 2 ? Pz - kz : kz;
@@ -349,7 +366,15 @@ __global__ void __launch_bounds__(4 * NPAR * Line<L>::T, YShape<L, NPAR>::minb) 
             if (kx < a.Hx) cpa4(Ks + e, karr(s) + kern_idx(a, kzm, r >> 2, kx, HY));
             else Ks[e] = 0.f;
         }
-        cpa_commit();
+    }
+    tw_copy(tw, a.fy.tw, P, tid, NT);
+    pdl_wait();
+    pdl_trigger();
+    if (inst_inactive(a, ib)) {  // (not before the copies in flight have landed)
+        cpa_wait_all();
+        __syncthreads();
+        for (int it = 0; a.Kblocked && it < 2 * kTileWaitLimit && !mbar_try_wait(&kbar, 0); it++) {}
+        return;
     }
     const long cs = (long)Pz * Ny * a.Lx;
     float2* col = inst_spec(a, ib) + ((long)kz * a.Lx + kx0) * Ny + w;
@@ -364,8 +389,8 @@ __global__ void __launch_bounds__(4 * NPAR * Line<L>::T, YShape<L, NPAR>::minb) 
                 v[c][q * LN::R1 + m] =
                     p2((LN::B1 % T == 0 || b < LN::B1) && y < Ny ? col[c * cs + 4 * y] : make_float2(0.f, 0.f));
             }
-    tw_copy(tw, a.fy.tw, P, tid, NT);
-    __syncthreads();  // twiddles, barrier initialised
+    cpa_wait_all();
+    __syncthreads();  // twiddles and caller-owned rows are here, barrier initialised
     float2* exl = ex + (w + 4 * p) * S::LS;
     line_fwd<LN, NPAR, 3, S::NBUF>(v, t, p, exl, S::lines * S::LS, tw);
     if (a.Kblocked) {
@@ -373,9 +398,6 @@ __global__ void __launch_bounds__(4 * NPAR * Line<L>::T, YShape<L, NPAR>::minb) 
             if (it == kTileWaitLimit && tid == 0) pass_timeout(a, ib);
             if (it >= 2 * kTileWaitLimit) return;
         }
-    } else {
-        cpa_wait_all();
-        __syncthreads();
     }
     // kernel multiply (kernmulrsymm3d.cl:41-90), ky mirrored into the stored
     // block; conjugated products: the inverse is conj(FFT(conj(.)))

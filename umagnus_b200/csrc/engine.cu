@@ -30,7 +30,7 @@ constexpr double kBoltzmann = 1.380650424e-23;  // mag/constants.go:9 Kb
 
 struct DevCtl {
     float* m;        // state magnetisation (3N, SoA)
-    float* mw;       // working / stage magnetisation
+    float* mw[2];    // working / stage magnetisations
     float* k[7];     // stage torques
     float* bd;       // demag field of this instance (batched ensembles)
     double t, dt, t0, alarm, stop;
@@ -38,6 +38,7 @@ struct DevCtl {
     int active;      // 0: the step in progress is skipped (stop time reached)
     unsigned int err2, dm2, rel;  // float bit patterns, atomicMax targets
     int nan_seen;
+    unsigned arrived;  // CTAs of the step's last torque kernel that are done
     int accepted;
     double last_err, peak_err, last_torque;
     long long nsteps, nundone, nevals;
@@ -75,7 +76,7 @@ struct LocalArgs {
     Mesh3 g;
     int N;
     DevCtl* ctl;
-    int m_sel;           // 0: ctl->m, 1: ctl->mw
+    int m_sel;           // 0: ctl->m, 1 and 2: ctl->mw[0] and [1]
     int out_slot;        // torque -> ctl->k[out_slot]
     float* tau_direct;   // if set, torque goes here instead
     float* beff;         // optional B_eff output
@@ -104,7 +105,8 @@ struct LocalArgs {
     const float* Ms;
     float Ms_mul;
     const InstParams* ip;  // batched: per-instance parameters (uniform maps only)
-    const float* mbuf1;    // the second magnetisation buffer (selects the tile map)
+    int early;             // demag passes precede the kernel: only its demag field has to be waited for
+    const float* mbuf[2];  // the second and third magnetisation buffers (select the tile map)
 };
 
 __global__ void k_local_consts(LocalArgs a, LocalConsts* out) {
@@ -150,360 +152,6 @@ __global__ void k_dmi_pairs(const float* __restrict__ aLUT, const float* __restr
     }
 }
 
-__device__ __forceinline__ f3 lltorque_g(f3 m, f3 H, float alpha, float gilb) {
-    f3 mxH = cross3(m, H);
-    f3 mmxH = cross3(m, mxH);
-    return f3{fm(gilb, fa(mxH.x, fm(alpha, mmxH.x))), fm(gilb, fa(mxH.y, fm(alpha, mmxH.y))),
-              fm(gilb, fa(mxH.z, fm(alpha, mmxH.z)))};
-}
-
-// engine/effectivefield.go:14-24 + engine/torque.go:135-144 for one cell:
-// B = demag; B += exchange(+DMI)/Ms; B += anisotropy; B += B_ext; torque.
-// UREG: every cell is in region 0 (no region map), so the region-pair
-// coefficients are scalars and no region is loaded.  TILE (with UREG, not
-// BAT, non-periodic mesh): the CTA's magnetisation tile with its halo comes
-// into shared memory by one TMA load (tile.cuh) and the stencils read it.
-// UNI (with UREG, not BAT): a uniform material with only the common terms --
-// uniform Ms, alpha and anisotropy, precession on, no OpenBC, and no
-// NoDemagSpins, bulk DMI, cubic anisotropy, thermal field, FreezeSpins or
-// B_eff output --
-// so that those tests and branches leave the instruction stream; the
-// arithmetic is the same operations in the same order.
-template <bool UREG, bool BAT, bool TILE, bool UNI = false>
-__global__ void __launch_bounds__(256) k_local_torque(const __grid_constant__ LocalArgs a,
-                                                      const __grid_constant__ TileMaps tm) {
-    static_assert(!TILE || (UREG && !BAT), "tiles: region-free, not batched");
-    static_assert(!UNI || (UREG && !BAT), "uniform material: region-free, not batched");
-    // BAT: blockIdx.z = iz + Nz * instance; the instance's controller,
-    // demag field and uniform parameters replace the shared ones
-    static_assert(!BAT || UREG, "batched ensembles have no region maps");
-    int iz = blockIdx.z;
-    DevCtl* ctl = a.ctl;
-    const float* bd = a.bd;
-    const LocalConsts* kcp = &a.kc;
-    float alpha_mul = a.alpha_mul;
-    const InstParams* ip = nullptr;
-    if constexpr (BAT) {
-        const int b = iz / a.g.Nz;
-        iz -= b * a.g.Nz;
-        ctl += b;
-        bd = ctl->bd;
-        ip = a.ip + b;
-        kcp = &ip->kc;
-        alpha_mul = ip->alpha_mul;
-    }
-    const LocalConsts& kc = *kcp;
-    const bool dmi = BAT ? ip->dmi != 0 : a.dmi != 0;
-    if (!ctl->active) return;
-    int ix = blockIdx.x * blockDim.x + threadIdx.x;
-    int iy = blockIdx.y * blockDim.y + threadIdx.y;
-    const int N = a.N;
-    const float* m = a.m_sel ? ctl->mw : ctl->m;
-    const float *mx = m, *my = m + N, *mz = m + 2 * N;
-    TileView tv{};
-    if constexpr (TILE) {
-        extern __shared__ __align__(128) float tile_raw[];
-        __shared__ __align__(8) uint64_t bar;
-        // the copy's destination on a 128-byte boundary whatever the offset of
-        // the dynamic region (launched with 128 bytes of slack)
-        float* const tile = tile_raw + ((128u - (smem_u32(tile_raw) & 127u)) & 127u) / sizeof(float);
-        const bool three_d = a.g.Nz > 1;
-        const uint32_t bytes = (uint32_t)tile_bytes(blockDim.x, blockDim.y, a.g.Nz);
-        const bool leader = threadIdx.x == 0 && threadIdx.y == 0;
-        if (leader) mbar_init(&bar, 1);
-        __syncthreads();
-        if (leader) {
-            mbar_expect_tx(&bar, bytes);
-            tma_load_4d(tile, &tm.map[m == a.mbuf1 ? 1 : 0], (int)(blockIdx.x * blockDim.x) - kTileHaloX,
-                        (int)(blockIdx.y * blockDim.y) - 1, three_d ? iz - 1 : iz, 0, &bar);
-        }
-        // bounded wait: past the limit flag the failure, wait once more for
-        // the copy in flight, and leave without writing
-        for (int it = 0; !mbar_try_wait(&bar, 0); it++) {
-            if (it == kTileWaitLimit && leader) atomicCAS(&ctl->status, 0, 7);
-            if (it >= 2 * kTileWaitLimit) return;
-        }
-        tv = TileView{tile, tile_pitch(blockDim.x), tile_rows(blockDim.y), three_d ? 3 : 1, three_d ? 1 : 0};
-    }
-    if (ix >= a.g.Nx || iy >= a.g.Ny) return;
-    int I = (iz * a.g.Ny + iy) * a.g.Nx + ix;
-    f3 B{0.f, 0.f, 0.f};
-    if (bd) B = f3{__ldg(bd + I), __ldg(bd + N + I), __ldg(bd + 2 * N + I)};
-    // engine/demag.go:95-97: NoDemagSpins cells feel no demag field
-    if (!BAT && !UNI && a.nodemag && __ldg(a.nodemag + (UREG ? 0 : __ldg(a.regions + I))) != 0.0f) B = f3{0.f, 0.f, 0.f};
-    f3 m0;
-    if constexpr (TILE) m0 = tv.at(threadIdx.x, threadIdx.y, 0, 0, 0);
-    else m0 = ld3(mx, my, mz, I);
-    if (!is0(m0)) {
-        f3 e;
-        if constexpr (TILE) {
-            e = dmi ? dmi_sum_tile<UNI>(tv, threadIdx.x, threadIdx.y, kc.pc, a.openbc != 0, a.g.Nz > 1, m0)
-                    : exchange_sum_tile(tv, threadIdx.x, threadIdx.y, kc.pc, a.g.Nz > 1, m0);
-        } else if (!BAT && !UNI && a.dbLUT) {  // engine/exchange.go:60-61 AddDMIBulk
-            e = dmibulk_sum(mx, my, mz, a.aLUT, a.dbLUT, a.regions, a.cx, a.cy, a.cz, a.g, a.openbc != 0, ix, iy,
-                            iz, m0, UREG ? 0 : __ldg(a.regions + I));
-        } else if constexpr (UREG) {
-            e = dmi ? dmi_sum_u(mx, my, mz, kc.pc, a.g, a.openbc != 0, ix, iy, iz, m0)
-                    : exchange_sum_u(mx, my, mz, kc.pc, a.g, ix, iy, iz, m0);
-        } else {
-            int r0 = __ldg(a.regions + I);
-            e = a.dmi ? dmi_sum_lut(mx, my, mz, a.dl, a.regions, a.g, a.openbc != 0, ix, iy, iz, m0, r0)
-                      : exchange_sum(mx, my, mz, a.aLUT, a.regions, a.wx, a.wy, a.wz, a.g, ix, iy, iz, m0, r0);
-        }
-        float inv = (BAT || UNI || a.ms_uniform) ? kc.inv_ms : inv_msat(a.Ms, a.Ms_mul, I);
-        B.x = fa(B.x, fm(e.x, inv));
-        B.y = fa(B.y, fm(e.y, inv));
-        B.z = fa(B.z, fm(e.z, inv));
-    }
-    if (a.anis) {
-        if (BAT || UNI || a.anis_uniform) {  // uniaxialanisotropy2.cl:27-34 with the uniform factors hoisted
-            f3 u{kc.u[0], kc.u[1], kc.u[2]};
-            float mu = dot3(m0, u);
-            float f1 = fm(kc.f1k, mu);
-            float f2 = fm(kc.f2k, fm(fm(mu, mu), mu));
-            B.x = fa(B.x, fa(fm(f1, u.x), fm(f2, u.x)));
-            B.y = fa(B.y, fa(fm(f1, u.y), fm(f2, u.y)));
-            B.z = fa(B.z, fa(fm(f1, u.z), fm(f2, u.z)));
-        } else {
-            add_uniaxial(B, a.up, m0, I);
-        }
-    }
-    if (!BAT && !UNI && a.cubic) add_cubic(B, a.cp, m0, I);  // engine/anisotropy.go:158
-    if (a.zeeman) {
-        if constexpr (BAT) {
-            B.x = fa(B.x, ip->bext[0]);
-            B.y = fa(B.y, ip->bext[1]);
-            B.z = fa(B.z, ip->bext[2]);
-        } else {
-            const int r = UREG ? 0 : __ldg(a.regions + I);
-            B.x = fa(B.x, __ldg(a.bext[0] + r));
-            B.y = fa(B.y, __ldg(a.bext[1] + r));
-            B.z = fa(B.z, __ldg(a.bext[2] + r));
-        }
-    }
-    if (!BAT && !UNI && a.thermal) {  // engine/effectivefield.go:20-22 B_therm (temperature2.cl)
-        const float sc = therm_scale(ctl->k2, amul(a.alpha, a.alpha_mul, I), amul(a.temp, a.temp_mul, I),
-                                     inv_msat(a.Ms, a.Ms_mul, I));
-        const f3 n = therm_normals(a.seed, ctl->nsteps, I);
-        B.x = fa(B.x, fm(n.x, sc));
-        B.y = fa(B.y, fm(n.y, sc));
-        B.z = fa(B.z, fm(n.z, sc));
-    }
-    if (!UNI && a.beff) { a.beff[I] = B.x; a.beff[N + I] = B.y; a.beff[2 * N + I] = B.z; }
-    f3 t;
-    if (!UNI && !a.precess) t = llnoprecess(m0, B);
-    else if (BAT || UNI || a.alpha_uniform) t = lltorque_g(m0, B, alpha_mul, kc.gilb);
-    else t = lltorque(m0, B, amul(a.alpha, a.alpha_mul, I));
-    // engine/torque.go:348-352 FreezeSpins (zeromask.cl)
-    if (!BAT && !UNI && a.frozen && __ldg(a.frozen + (UREG ? 0 : __ldg(a.regions + I))) != 0.0f) t = f3{0.f, 0.f, 0.f};
-    float* out = a.tau_direct ? a.tau_direct : ctl->k[a.out_slot];
-    out[I] = t.x; out[N + I] = t.y; out[2 * N + I] = t.z;
-}
-
-// ---------------------------------------------------------------- stages
-constexpr int kMaxTerms = 7;
-struct StageArgs {
-    DevCtl* ctl;
-    int N;
-    int nterm;
-    int src_m;             // first term: 0 = ctl->m, 1 = ctl->mw (coefficient 1)
-    int slot[kMaxTerms];   // k slots of terms 1..nterm-1
-    float c[kMaxTerms];    // float32 constants multiplying h (terms 1..)
-    int scale_h;           // 1: fac = c*h ; 0: fac = c
-    int normalize;
-    int only_if_accepted;  // RK4 final solution
-    const float* vol;
-};
-
-// m_w = normalize(src + sum_j (c_j h) k_j) with Madd<n> rounding
-// (opencl/madd.go, madd<n>.cl) then normalize2.cl.  NT = number of terms.
-template <int NT, bool BAT>
-__global__ void __launch_bounds__(256) k_stage(StageArgs a) {
-    DevCtl* ctl = a.ctl + (BAT ? blockIdx.y : 0);  // BAT: one grid row per instance
-    if (!ctl->active) return;
-    if (a.only_if_accepted && !ctl->accepted) return;
-    const float h = ctl->h;
-    float fac[NT];
-    const float* src[NT];
-    fac[0] = 1.0f;
-    src[0] = a.src_m ? ctl->mw : ctl->m;
-#pragma unroll
-    for (int j = 1; j < NT; j++) {
-        fac[j] = a.scale_h ? fm(a.c[j], h) : a.c[j];
-        src[j] = ctl->k[a.slot[j]];
-    }
-    float* dst = ctl->mw;
-    const int N = a.N;
-    // one component of one cell from its NT source values (Madd<NT> order)
-    auto comb = [&](const float (&x)[NT]) {
-        if constexpr (NT == 3) {
-            return fa(fm(fac[0], x[0]), fa(fm(fac[1], x[1]), fm(fac[2], x[2])));
-        } else {
-            float acc = fm(fac[0], x[0]);
-#pragma unroll
-            for (int j = 1; j < NT; j++) acc = fa(acc, fm(fac[j], x[j]));
-            return acc;
-        }
-    };
-    auto finish = [&](float (&v)[3], float w) {
-        if (a.normalize) {
-            f3 r = normalize_vol(f3{v[0], v[1], v[2]}, w);
-            v[0] = r.x; v[1] = r.y; v[2] = r.z;
-        }
-    };
-    // Four cells per iteration with 16-byte loads and stores where every
-    // array allows it (N a multiple of 4, 16-byte aligned bases): four times
-    // the bytes in flight per thread; each cell's arithmetic is unchanged.
-    bool vec = (N & 3) == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0 &&
-               (!a.vol || (reinterpret_cast<uintptr_t>(a.vol) & 15) == 0);
-#pragma unroll
-    for (int j = 0; j < NT; j++) vec = vec && (reinterpret_cast<uintptr_t>(src[j]) & 15) == 0;
-    if (vec) {
-        const int N4 = N >> 2;
-        for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < N4; q += gridDim.x * blockDim.x) {
-            float v[4][3];
-#pragma unroll
-            for (int c = 0; c < 3; c++) {
-                float4 x4[NT];
-#pragma unroll
-                for (int j = 0; j < NT; j++) x4[j] = reinterpret_cast<const float4*>(src[j] + (size_t)c * N)[q];
-#pragma unroll
-                for (int l = 0; l < 4; l++) {
-                    float x[NT];
-#pragma unroll
-                    for (int j = 0; j < NT; j++) x[j] = l == 0 ? x4[j].x : l == 1 ? x4[j].y : l == 2 ? x4[j].z : x4[j].w;
-                    v[l][c] = comb(x);
-                }
-            }
-            const float4 w4 = a.vol ? reinterpret_cast<const float4*>(a.vol)[q] : make_float4(1.f, 1.f, 1.f, 1.f);
-            finish(v[0], w4.x);
-            finish(v[1], w4.y);
-            finish(v[2], w4.z);
-            finish(v[3], w4.w);
-#pragma unroll
-            for (int c = 0; c < 3; c++)
-                reinterpret_cast<float4*>(dst + (size_t)c * N)[q] = make_float4(v[0][c], v[1][c], v[2][c], v[3][c]);
-        }
-        return;
-    }
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
-        float v[3];
-#pragma unroll
-        for (int c = 0; c < 3; c++) {
-            float x[NT];
-#pragma unroll
-            for (int j = 0; j < NT; j++) x[j] = src[j][c * N + i];
-            v[c] = comb(x);
-        }
-        finish(v, a.vol ? a.vol[i] : 1.0f);
-        dst[i] = v[0]; dst[N + i] = v[1]; dst[2 * N + i] = v[2];
-    }
-}
-
-// ---------------------------------------------------------------- error norms
-struct ErrArgs {
-    DevCtl* ctl;
-    int N;
-    int nterm;
-    int slot[kMaxTerms];
-    float e[kMaxTerms];
-    int dm_slot;     // slot whose max norm is the torque of the new state (delM / k4 / dy)
-    int heun;        // 1: error = |k[slot0] - k[slot1]| (MaxVecDiff)
-};
-
-// Fused: error combination (Madd rounding), max |Err|^2, max |delM|^2 and
-// max |Err|/|delM| (VecNorm + Div + MaxAbs of stepcontroller.go:51-63);
-// Err itself is never written to memory.
-template <int NT, bool HEUN, bool BAT>
-__global__ void __launch_bounds__(256) k_err_norms(ErrArgs a) {
-    __shared__ float sh[32];
-    DevCtl* ctl = a.ctl + (BAT ? blockIdx.y : 0);  // BAT: one grid row per instance
-    if (!ctl->active) return;
-    const float* k[NT];
-    float e[NT];
-#pragma unroll
-    for (int j = 0; j < NT; j++) {
-        k[j] = ctl->k[a.slot[j]];
-        e[j] = a.e[j];
-    }
-    const float* dm = ctl->k[a.dm_slot];
-    const int N = a.N;
-    float me = 0.f, md = 0.f, mr = 0.f;
-    int nan = 0;
-    // one component of the error estimate of one cell (Madd<NT> order)
-    auto comb = [&](const float (&x)[NT]) {
-        if constexpr (HEUN) {
-            return fs(x[0], x[1]);
-        } else if constexpr (NT == 3) {
-            return fa(fm(e[0], x[0]), fa(fm(e[1], x[1]), fm(e[2], x[2])));
-        } else {
-            float acc = fm(e[0], x[0]);
-#pragma unroll
-            for (int j = 1; j < NT; j++) acc = fa(acc, fm(e[j], x[j]));
-            return acc;
-        }
-    };
-    auto cell = [&](f3 E, f3 D) {
-        float e2 = dot3(E, E), d2 = dot3(D, D);
-        float en = __fsqrt_rn(e2), dn = __fsqrt_rn(d2);
-        float r = dn == 0.0f ? 0.0f : fd(en, dn);
-        nan |= (e2 != e2) | (d2 != d2);
-        me = fmaxf(me, e2);
-        md = fmaxf(md, d2);
-        mr = fmaxf(mr, r);
-    };
-    // four cells per iteration with 16-byte loads where every array allows
-    // it (the maxima do not depend on the order cells are visited in)
-    bool vec = (N & 3) == 0 && (reinterpret_cast<uintptr_t>(dm) & 15) == 0;
-#pragma unroll
-    for (int j = 0; j < NT; j++) vec = vec && (reinterpret_cast<uintptr_t>(k[j]) & 15) == 0;
-    if (vec) {
-        const int N4 = N >> 2;
-        for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < N4; q += gridDim.x * blockDim.x) {
-            float E[4][3], D[4][3];
-#pragma unroll
-            for (int c = 0; c < 3; c++) {
-                float4 x4[NT];
-#pragma unroll
-                for (int j = 0; j < NT; j++) x4[j] = reinterpret_cast<const float4*>(k[j] + (size_t)c * N)[q];
-                const float4 d4 = reinterpret_cast<const float4*>(dm + (size_t)c * N)[q];
-                D[0][c] = d4.x; D[1][c] = d4.y; D[2][c] = d4.z; D[3][c] = d4.w;
-#pragma unroll
-                for (int l = 0; l < 4; l++) {
-                    float x[NT];
-#pragma unroll
-                    for (int j = 0; j < NT; j++) x[j] = l == 0 ? x4[j].x : l == 1 ? x4[j].y : l == 2 ? x4[j].z : x4[j].w;
-                    E[l][c] = comb(x);
-                }
-            }
-#pragma unroll
-            for (int l = 0; l < 4; l++) cell(f3{E[l][0], E[l][1], E[l][2]}, f3{D[l][0], D[l][1], D[l][2]});
-        }
-    } else {
-        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
-            float Ec[3];
-#pragma unroll
-            for (int c = 0; c < 3; c++) {
-                float x[NT];
-#pragma unroll
-                for (int j = 0; j < NT; j++) x[j] = k[j][c * N + i];
-                Ec[c] = comb(x);
-            }
-            cell(f3{Ec[0], Ec[1], Ec[2]}, f3{dm[i], dm[N + i], dm[2 * N + i]});
-        }
-    }
-    me = block_max<256>(me, sh);
-    md = block_max<256>(md, sh);
-    mr = block_max<256>(mr, sh);
-    nan = __syncthreads_or(nan);
-    if (threadIdx.x == 0) {
-        atomic_max_nonneg(&ctl->err2, me);
-        atomic_max_nonneg(&ctl->dm2, md);
-        atomic_max_nonneg(&ctl->rel, mr);
-        if (nan) atomicOr(&ctl->nan_seen, 1);
-    }
-}
-
 // ---------------------------------------------------------------- controller
 __device__ void adapt_dt(DevCtl* c, double corr) {
     if (c->fix_dt != 0) { c->dt = c->fix_dt; return; }
@@ -526,30 +174,45 @@ __device__ void adapt_dt(DevCtl* c, double corr) {
 
 // engine/rk45dp.go:16-50 (start of Step): fixed dt, h, t0, clear maxima;
 // skip the step once the run's stop time is reached (engine/run.go:212-231).
-__global__ void k_step_begin(DevCtl* c0, int nb) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;  // one thread per instance
-    if (b >= nb) return;
-    DevCtl* c = c0 + b;
-    c->active = (c->t < c->stop) && c->status == 0;
+// Every CTA of a first stage kernel evaluates step_runs and step_h; one of
+// its threads also runs step_begin, which changes nothing that they read.
+__device__ __forceinline__ bool step_runs(const DevCtl* c) { return c->t < c->stop && c->status == 0; }
+__device__ __forceinline__ float step_h(const DevCtl* c) {
+    return (float)((c->fix_dt != 0 ? c->fix_dt : c->dt) * c->gamma);
+}
+__device__ __forceinline__ void step_begin(DevCtl* c) {
+    c->active = step_runs(c);
     if (!c->active) return;
     if (c->fix_dt != 0) c->dt = c->fix_dt;
     c->h = (float)(c->dt * c->gamma);
     if (c->therm_gv != 0) c->k2 = (float)(2 * kBoltzmann / (c->therm_gv * c->dt));
     c->t0 = c->t;
     c->err2 = 0u; c->dm2 = 0u; c->rel = 0u;
+    c->arrived = 0u;
     c->accepted = 0;
 }
+__global__ void k_step_begin(DevCtl* c0, int nb) {
+    const int b = blockIdx.x * blockDim.x + threadIdx.x;  // one thread per instance
+    pdl_wait();
+    pdl_trigger();
+    if (b < nb) step_begin(c0 + b);
+}
+
+// what the controller of a stepper does after its last evaluation
+struct CtlArgs {
+    int kind, acc, rej;      // controller and its exponents, below
+    int fsal_from, fsal_to;  // k slots swapped on acceptance (-1: none)
+    int nevals;
+    int new_m;               // the working buffer (1, 2) that becomes the state
+    int rk4;                 // record max |k4| (setMaxTorque, engine/rk4.go:64)
+};
 
 // kind 0: integralController (engine/stepcontroller.go:35-97), FSAL when fsal
 // kind 1: simpleController (:13-32, RK4); kind 2: Heun (engine/heun.go:40-58)
 // kind 3: Euler (engine/euler.go:16-35), always accepted
-__global__ void k_controller(DevCtl* c0, int nb, int kind, int acc, int rej, int fsal_from, int fsal_to,
-                             int nevals) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;  // one thread per instance
-    if (b >= nb) return;
-    DevCtl* c = c0 + b;
-    if (!c->active) return;
-    c->nevals += nevals;
+__device__ void controller(DevCtl* c, const CtlArgs& q) {
+    const int kind = q.kind, acc = q.acc, rej = q.rej;
+    c->nevals += q.nevals;
     if (c->nan_seen) c->status = 4;
     if (kind == 3) {
         // setMaxTorque(dy0), then dt = FixDt, or float32(MaxErr / LastTorque)
@@ -636,26 +299,541 @@ __global__ void k_controller(DevCtl* c0, int nb, int kind, int acc, int rej, int
             adapt_dt(c, pow(c->max_err / err, 1. / 3.));
         }
     }
-    if (c->accepted && kind == 0 && fsal_from >= 0) {
-        float* t = c->k[fsal_to];
-        c->k[fsal_to] = c->k[fsal_from];
-        c->k[fsal_from] = t;
+    if (c->accepted && kind == 0 && q.fsal_from >= 0) {
+        float* t = c->k[q.fsal_to];
+        c->k[q.fsal_to] = c->k[q.fsal_from];
+        c->k[q.fsal_from] = t;
     }
 }
 
-// accepted: the working magnetisation becomes the state (pointer swap);
-// RK4 also records max |k4| here (setMaxTorque, engine/rk4.go:64)
-__global__ void k_step_end(DevCtl* c0, int nb, int rk4) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;  // one thread per instance
-    if (b >= nb) return;
-    DevCtl* c = c0 + b;
-    if (!c->active) return;
+// Controller and end of the step, by one thread once every CTA of the step's
+// last evaluation has added its maxima.  Accepted: the working
+// magnetisation becomes the state (pointer swap); the steppers that form
+// their solution afterwards (Euler, Heun, RK4) write it to the new state
+// buffer from the old one.
+__device__ __noinline__ void step_finish(DevCtl* c, const CtlArgs& q) {
+    // other CTAs' atomics: read past this SM's L1
+    c->err2 = __ldcg(&c->err2);
+    c->dm2 = __ldcg(&c->dm2);
+    c->rel = __ldcg(&c->rel);
+    c->nan_seen = __ldcg(&c->nan_seen);
+    controller(c, q);
     if (c->accepted) {
         float* t = c->m;
-        c->m = c->mw;
-        c->mw = t;
-        if (rk4) c->last_torque = sqrt((double)__uint_as_float(c->dm2));
+        c->m = c->mw[q.new_m - 1];
+        c->mw[q.new_m - 1] = t;
+        if (q.rk4) c->last_torque = sqrt((double)__uint_as_float(c->dm2));
     }
+}
+
+// ---------------------------------------------------------------- after an evaluation
+constexpr int kMaxTerms = 7;
+// What the torque kernel does with a cell's torque besides storing it (or, where
+// fuse_tails says so, kernels of their own).
+// kStage: the next working magnetisation, dst = normalize(m + sum_j (c_j h)
+// k_j) with Madd<n> rounding (opencl/madd.go, madd<n>.cl) then normalize2.cl;
+// the cell's own torque is the last term.  kErr: the error estimate
+// sum_j e_j k_j and its maxima, again with the torque as the last term; the
+// last CTA to finish runs the controller.
+enum { kNoTail = 0, kStageTail = 1, kErrTail = 2 };
+struct TailArgs {
+    int kind = kNoTail;
+    int nk = 0;              // stored torques that take part
+    int slot[kMaxTerms];
+    float c[kMaxTerms];      // float32 constants of those and (at nk) of the cell's own torque
+    int dst = 0;             // stage: 1 or 2, ctl->mw
+    int normalize = 0;
+    const float* vol = nullptr;
+    int heun = 0;            // error = |k - own| (MaxVecDiff)
+    CtlArgs ctl{};
+};
+__device__ __forceinline__ float* mbuf(const DevCtl* c, int sel) { return sel == 0 ? c->m : c->mw[sel - 1]; }
+
+// Values a cell's tail needs from memory; requested before the stencil, so
+// that they arrive while the field is summed.
+struct TailIn {
+    f3 m, k[5];
+    float vol;
+};
+template <int TAIL> __device__ __forceinline__ void tail_load(TailIn& in, const TailArgs& ta, const DevCtl* ctl, int N, int I) {
+    if constexpr (TAIL != kNoTail) {
+#pragma unroll
+        for (int j = 0; j < 5; j++)
+            if (j < ta.nk) {
+                const float* k = ctl->k[ta.slot[j]];
+                in.k[j] = f3{k[I], k[N + I], k[2 * N + I]};
+            }
+    }
+    if constexpr (TAIL == kStageTail) {
+        in.m = f3{ctl->m[I], ctl->m[N + I], ctl->m[2 * N + I]};
+        in.vol = ta.vol ? __ldg(ta.vol + I) : 1.0f;
+    }
+}
+// one component of the stage (x: values of the terms nk.., factors fac)
+__device__ __forceinline__ float stage_comb(int nk, const float (&fac)[6], float m, const float (&k)[5], float t) {
+    if (nk == 1) return fa(fm(1.0f, m), fa(fm(fac[0], k[0]), fm(fac[1], t)));  // madd3
+    float acc = fm(1.0f, m);
+    float ft = fac[0];
+#pragma unroll
+    for (int j = 0; j < 5; j++)
+        if (j < nk) {
+            acc = fa(acc, fm(fac[j], k[j]));
+            ft = fac[j + 1];
+        }
+    return fa(acc, fm(ft, t));
+}
+__device__ __forceinline__ void stage_tail(const TailIn& in, const TailArgs& ta, const DevCtl* ctl, int N, int I, f3 t) {
+    const float h = ctl->h;
+    float fac[6];
+#pragma unroll
+    for (int j = 0; j < 6; j++) fac[j] = fm(ta.c[j], h);
+    const float kx[5] = {in.k[0].x, in.k[1].x, in.k[2].x, in.k[3].x, in.k[4].x};
+    const float ky[5] = {in.k[0].y, in.k[1].y, in.k[2].y, in.k[3].y, in.k[4].y};
+    const float kz[5] = {in.k[0].z, in.k[1].z, in.k[2].z, in.k[3].z, in.k[4].z};
+    f3 v{stage_comb(ta.nk, fac, in.m.x, kx, t.x), stage_comb(ta.nk, fac, in.m.y, ky, t.y),
+         stage_comb(ta.nk, fac, in.m.z, kz, t.z)};
+    if (ta.normalize) v = normalize_vol(v, in.vol);
+    float* d = mbuf(ctl, ta.dst);
+    d[I] = v.x; d[N + I] = v.y; d[2 * N + I] = v.z;
+}
+// max |Err|^2, max |delM|^2 and max |Err|/|delM| of one cell (VecNorm + Div +
+// MaxAbs of stepcontroller.go:51-63); Err itself is never written to memory.
+// NaNs are ignored like the reference's fmax and reported apart.
+struct ErrMax {
+    float e2 = 0.f, d2 = 0.f, rel = 0.f;
+    int nan = 0;
+};
+__device__ __forceinline__ ErrMax err_tail(const TailIn& in, const TailArgs& ta, f3 t) {
+    auto comb = [&](const float (&k)[5], float x) {
+        if (ta.heun) return fs(ta.nk ? k[0] : x, x);
+        float acc = fm(ta.c[0], k[0]), ct = ta.c[1];
+#pragma unroll
+        for (int j = 1; j < 5; j++)
+            if (j < ta.nk) {
+                acc = fa(acc, fm(ta.c[j], k[j]));
+                ct = ta.c[j + 1];
+            }
+        return fa(acc, fm(ct, x));
+    };
+    const float kx[5] = {in.k[0].x, in.k[1].x, in.k[2].x, in.k[3].x, in.k[4].x};
+    const float ky[5] = {in.k[0].y, in.k[1].y, in.k[2].y, in.k[3].y, in.k[4].y};
+    const float kz[5] = {in.k[0].z, in.k[1].z, in.k[2].z, in.k[3].z, in.k[4].z};
+    const f3 E{comb(kx, t.x), comb(ky, t.y), comb(kz, t.z)};
+    const float e2 = dot3(E, E), d2 = dot3(t, t);
+    const float en = __fsqrt_rn(e2), dn = __fsqrt_rn(d2);
+    const float r = dn == 0.0f ? 0.0f : fd(en, dn);
+    return ErrMax{fmaxf(0.f, e2), fmaxf(0.f, d2), fmaxf(0.f, r), (e2 != e2) | (d2 != d2)};
+}
+// The CTA's maxima to the controller record; the last of the instance's ncta
+// CTAs then runs the controller.  Whole warps (block sizes are multiples of 32).
+// The record is read before it is updated: maxima settle after a few CTAs, and
+// tens of thousands of atomics on one address would bound a large mesh.
+__device__ __forceinline__ void err_finish(const ErrMax& v, bool ok, const TailArgs& ta, DevCtl* ctl, unsigned ncta) {
+    __shared__ unsigned sh[4][8];
+    const int tid = threadIdx.y * blockDim.x + threadIdx.x, nw = (blockDim.x * blockDim.y) >> 5;
+    const unsigned e = __reduce_max_sync(0xffffffffu, __float_as_uint(v.e2));
+    const unsigned d = __reduce_max_sync(0xffffffffu, __float_as_uint(v.d2));
+    const unsigned r = __reduce_max_sync(0xffffffffu, __float_as_uint(v.rel));
+    const unsigned n = __reduce_or_sync(0xffffffffu, (unsigned)v.nan | (ok ? 0u : 2u));
+    if ((tid & 31) == 0) {
+        sh[0][tid >> 5] = e; sh[1][tid >> 5] = d; sh[2][tid >> 5] = r; sh[3][tid >> 5] = n;
+    }
+    __syncthreads();  // (and every read of the record by this CTA is done)
+    if (tid != 0) return;
+    unsigned me = 0, md = 0, mr = 0, mn = 0;
+    for (int w = 0; w < nw; w++) {
+        me = max(me, sh[0][w]); md = max(md, sh[1][w]); mr = max(mr, sh[2][w]); mn |= sh[3][w];
+    }
+    if (me > __ldcg(&ctl->err2)) atomicMax(&ctl->err2, me);
+    if (md > __ldcg(&ctl->dm2)) atomicMax(&ctl->dm2, md);
+    if (mr > __ldcg(&ctl->rel)) atomicMax(&ctl->rel, mr);
+    if (mn & 1) atomicOr(&ctl->nan_seen, 1);
+    if (mn & 2) return;  // a wait gave up: the status says so, and the step does not end
+    __threadfence();
+    if (atomicAdd(&ctl->arrived, 1u) + 1u == ncta) {
+        __threadfence();
+        step_finish(ctl, ta.ctl);
+    }
+}
+
+__device__ __forceinline__ f3 lltorque_g(f3 m, f3 H, float alpha, float gilb) {
+    f3 mxH = cross3(m, H);
+    f3 mmxH = cross3(m, mxH);
+    return f3{fm(gilb, fa(mxH.x, fm(alpha, mmxH.x))), fm(gilb, fa(mxH.y, fm(alpha, mmxH.y))),
+              fm(gilb, fa(mxH.z, fm(alpha, mmxH.z)))};
+}
+
+// engine/effectivefield.go:14-24 + engine/torque.go:135-144 for one cell:
+// B = demag; B += exchange(+DMI)/Ms; B += anisotropy; B += B_ext; torque.
+// UREG: every cell is in region 0 (no region map), so the region-pair
+// coefficients are scalars and no region is loaded.  TILE (with UREG, not
+// BAT, non-periodic mesh): the CTA's magnetisation tile with its halo comes
+// into shared memory by one TMA load (tile.cuh) and the stencils read it.
+// UNI (with UREG, not BAT): a uniform material with only the common terms --
+// uniform Ms, alpha and anisotropy, precession on, no OpenBC, and no
+// NoDemagSpins, bulk DMI, cubic anisotropy, thermal field, FreezeSpins or
+// B_eff output --
+// so that those tests and branches leave the instruction stream; the
+// arithmetic is the same operations in the same order.
+template <bool UREG, bool BAT, bool TILE, bool UNI, int TAIL>
+__global__ void __launch_bounds__(256) k_local_torque(const __grid_constant__ LocalArgs a,
+                                                      const __grid_constant__ TileMaps tm,
+                                                      const __grid_constant__ TailArgs ta) {
+    static_assert(!TILE || (UREG && !BAT), "tiles: region-free, not batched");
+    static_assert(!UNI || (UREG && !BAT), "uniform material: region-free, not batched");
+    // BAT: blockIdx.z = iz + Nz * instance; the instance's controller,
+    // demag field and uniform parameters replace the shared ones
+    static_assert(!BAT || UREG, "batched ensembles have no region maps");
+    // behind the demag passes everything but the demag field was written by
+    // kernels before the last one: it is loaded, and the stencil summed, while
+    // the last pass runs (common.cuh)
+    if (!a.early) {
+        pdl_wait();
+        pdl_trigger();
+    }
+    int iz = blockIdx.z;
+    DevCtl* ctl = a.ctl;
+    const float* bd = a.bd;
+    const LocalConsts* kcp = &a.kc;
+    float alpha_mul = a.alpha_mul;
+    const InstParams* ip = nullptr;
+    if constexpr (BAT) {
+        const int b = iz / a.g.Nz;
+        iz -= b * a.g.Nz;
+        ctl += b;
+        bd = ctl->bd;
+        ip = a.ip + b;
+        kcp = &ip->kc;
+        alpha_mul = ip->alpha_mul;
+    }
+    const LocalConsts& kc = *kcp;
+    const bool dmi = BAT ? ip->dmi != 0 : a.dmi != 0;
+    if (!ctl->active) {
+        pdl_wait();
+        return;
+    }
+    int ix = blockIdx.x * blockDim.x + threadIdx.x;
+    int iy = blockIdx.y * blockDim.y + threadIdx.y;
+    const int N = a.N;
+    const float* m = mbuf(ctl, a.m_sel);
+    const float *mx = m, *my = m + N, *mz = m + 2 * N;
+    TileView tv{};
+    bool live = true;  // the tile arrived
+    if constexpr (TILE) {
+        extern __shared__ __align__(128) float tile_raw[];
+        __shared__ __align__(8) uint64_t bar;
+        // the copy's destination on a 128-byte boundary whatever the offset of
+        // the dynamic region (launched with 128 bytes of slack)
+        float* const tile = tile_raw + ((128u - (smem_u32(tile_raw) & 127u)) & 127u) / sizeof(float);
+        const bool three_d = a.g.Nz > 1;
+        const uint32_t bytes = (uint32_t)tile_bytes(blockDim.x, blockDim.y, a.g.Nz);
+        const bool leader = threadIdx.x == 0 && threadIdx.y == 0;
+        if (leader) mbar_init(&bar, 1);
+        __syncthreads();
+        if (leader) {
+            mbar_expect_tx(&bar, bytes);
+            tma_load_4d(tile, &tm.map[m == a.mbuf[0] ? 1 : m == a.mbuf[1] ? 2 : 0], (int)(blockIdx.x * blockDim.x) - kTileHaloX,
+                        (int)(blockIdx.y * blockDim.y) - 1, three_d ? iz - 1 : iz, 0, &bar);
+        }
+        // bounded wait: past the limit flag the failure, wait once more for
+        // the copy in flight, and leave without writing
+        for (int it = 0; live && !mbar_try_wait(&bar, 0); it++) {
+            if (it == kTileWaitLimit && leader) atomicCAS(&ctl->status, 0, 7);
+            if (it >= 2 * kTileWaitLimit) live = false;
+        }
+        tv = TileView{tile, tile_pitch(blockDim.x), tile_rows(blockDim.y), three_d ? 3 : 1, three_d ? 1 : 0};
+    }
+    const bool cell = live && ix < a.g.Nx && iy < a.g.Ny;
+    if (!cell && a.early) pdl_wait();
+    if (TAIL != kErrTail && !cell) return;
+    ErrMax err{};
+    if (cell) {
+        int I = (iz * a.g.Ny + iy) * a.g.Nx + ix;
+        TailIn in{};
+        tail_load<TAIL>(in, ta, ctl, N, I);
+        f3 m0;
+        if constexpr (TILE) m0 = tv.at(threadIdx.x, threadIdx.y, 0, 0, 0);
+        else m0 = ld3(mx, my, mz, I);
+        const bool magnetic = !is0(m0);
+        f3 e{0.f, 0.f, 0.f};
+        float inv = 0.f;
+        if (magnetic) {
+            if constexpr (TILE) {
+                e = dmi ? dmi_sum_tile<UNI>(tv, threadIdx.x, threadIdx.y, kc.pc, a.openbc != 0, a.g.Nz > 1, m0)
+                        : exchange_sum_tile(tv, threadIdx.x, threadIdx.y, kc.pc, a.g.Nz > 1, m0);
+            } else if (!BAT && !UNI && a.dbLUT) {  // engine/exchange.go:60-61 AddDMIBulk
+                e = dmibulk_sum(mx, my, mz, a.aLUT, a.dbLUT, a.regions, a.cx, a.cy, a.cz, a.g, a.openbc != 0, ix, iy,
+                                iz, m0, UREG ? 0 : __ldg(a.regions + I));
+            } else if constexpr (UREG) {
+                e = dmi ? dmi_sum_u(mx, my, mz, kc.pc, a.g, a.openbc != 0, ix, iy, iz, m0)
+                        : exchange_sum_u(mx, my, mz, kc.pc, a.g, ix, iy, iz, m0);
+            } else {
+                int r0 = __ldg(a.regions + I);
+                e = a.dmi ? dmi_sum_lut(mx, my, mz, a.dl, a.regions, a.g, a.openbc != 0, ix, iy, iz, m0, r0)
+                          : exchange_sum(mx, my, mz, a.aLUT, a.regions, a.wx, a.wy, a.wz, a.g, ix, iy, iz, m0, r0);
+            }
+            inv = (BAT || UNI || a.ms_uniform) ? kc.inv_ms : inv_msat(a.Ms, a.Ms_mul, I);
+        }
+        if (a.early) {
+            pdl_wait();
+            pdl_trigger();
+        }
+        f3 B{0.f, 0.f, 0.f};
+        if (bd) B = f3{bd[I], bd[N + I], bd[2 * N + I]};
+        // engine/demag.go:95-97: NoDemagSpins cells feel no demag field
+        if (!BAT && !UNI && a.nodemag && __ldg(a.nodemag + (UREG ? 0 : __ldg(a.regions + I))) != 0.0f) B = f3{0.f, 0.f, 0.f};
+        if (magnetic) {
+            B.x = fa(B.x, fm(e.x, inv));
+            B.y = fa(B.y, fm(e.y, inv));
+            B.z = fa(B.z, fm(e.z, inv));
+        }
+        if (a.anis) {
+            if (BAT || UNI || a.anis_uniform) {  // uniaxialanisotropy2.cl:27-34 with the uniform factors hoisted
+                f3 u{kc.u[0], kc.u[1], kc.u[2]};
+                float mu = dot3(m0, u);
+                float f1 = fm(kc.f1k, mu);
+                float f2 = fm(kc.f2k, fm(fm(mu, mu), mu));
+                B.x = fa(B.x, fa(fm(f1, u.x), fm(f2, u.x)));
+                B.y = fa(B.y, fa(fm(f1, u.y), fm(f2, u.y)));
+                B.z = fa(B.z, fa(fm(f1, u.z), fm(f2, u.z)));
+            } else {
+                add_uniaxial(B, a.up, m0, I);
+            }
+        }
+        if (!BAT && !UNI && a.cubic) add_cubic(B, a.cp, m0, I);  // engine/anisotropy.go:158
+        if (a.zeeman) {
+            if constexpr (BAT) {
+                B.x = fa(B.x, ip->bext[0]);
+                B.y = fa(B.y, ip->bext[1]);
+                B.z = fa(B.z, ip->bext[2]);
+            } else {
+                const int r = UREG ? 0 : __ldg(a.regions + I);
+                B.x = fa(B.x, __ldg(a.bext[0] + r));
+                B.y = fa(B.y, __ldg(a.bext[1] + r));
+                B.z = fa(B.z, __ldg(a.bext[2] + r));
+            }
+        }
+        if (!BAT && !UNI && a.thermal) {  // engine/effectivefield.go:20-22 B_therm (temperature2.cl)
+            const float sc = therm_scale(ctl->k2, amul(a.alpha, a.alpha_mul, I), amul(a.temp, a.temp_mul, I),
+                                         inv_msat(a.Ms, a.Ms_mul, I));
+            const f3 n = therm_normals(a.seed, ctl->nsteps, I);
+            B.x = fa(B.x, fm(n.x, sc));
+            B.y = fa(B.y, fm(n.y, sc));
+            B.z = fa(B.z, fm(n.z, sc));
+        }
+        if (!UNI && a.beff) { a.beff[I] = B.x; a.beff[N + I] = B.y; a.beff[2 * N + I] = B.z; }
+        f3 t;
+        if (!UNI && !a.precess) t = llnoprecess(m0, B);
+        else if (BAT || UNI || a.alpha_uniform) t = lltorque_g(m0, B, alpha_mul, kc.gilb);
+        else t = lltorque(m0, B, amul(a.alpha, a.alpha_mul, I));
+        // engine/torque.go:348-352 FreezeSpins (zeromask.cl)
+        if (!BAT && !UNI && a.frozen && __ldg(a.frozen + (UREG ? 0 : __ldg(a.regions + I))) != 0.0f) t = f3{0.f, 0.f, 0.f};
+        float* out = a.tau_direct ? a.tau_direct : ctl->k[a.out_slot];
+        out[I] = t.x; out[N + I] = t.y; out[2 * N + I] = t.z;
+        if constexpr (TAIL == kStageTail) stage_tail(in, ta, ctl, N, I, t);
+        if constexpr (TAIL == kErrTail) err = err_tail(in, ta, t);
+    }
+    if constexpr (TAIL == kErrTail) err_finish(err, live, ta, ctl, gridDim.x * gridDim.y * (BAT ? a.g.Nz : gridDim.z));
+}
+
+// ---------------------------------------------------------------- stages
+struct StageArgs {
+    DevCtl* ctl;
+    int N;
+    int nterm;
+    int src, dst;          // first term (coefficient 1) and result: 0 = ctl->m, 1 and 2 = ctl->mw[0] and [1]
+    int slot[kMaxTerms];   // k slots of terms 1..nterm-1
+    float c[kMaxTerms];    // float32 constants multiplying h (terms 1..)
+    int normalize;
+    int begin;             // the step's first kernel: start the step
+    int only_if_accepted;  // the solution formed after the controller
+    const float* vol;
+};
+
+// dst = normalize(src + sum_j (c_j h) k_j) with Madd<n> rounding
+// (opencl/madd.go, madd<n>.cl) then normalize2.cl.  NT = number of terms.
+template <int NT, bool BAT>
+__global__ void __launch_bounds__(256) k_stage(StageArgs a) {
+    DevCtl* ctl = a.ctl + (BAT ? blockIdx.y : 0);  // BAT: one grid row per instance
+    pdl_wait();
+    pdl_trigger();
+    float h;
+    if (a.begin) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) step_begin(ctl);
+        if (!step_runs(ctl)) return;
+        h = step_h(ctl);
+    } else {
+        if (!ctl->active) return;
+        if (a.only_if_accepted && !ctl->accepted) return;
+        h = ctl->h;
+    }
+    float fac[NT];
+    const float* src[NT];
+    fac[0] = 1.0f;
+    src[0] = mbuf(ctl, a.src);
+#pragma unroll
+    for (int j = 1; j < NT; j++) {
+        fac[j] = fm(a.c[j], h);
+        src[j] = ctl->k[a.slot[j]];
+    }
+    float* dst = mbuf(ctl, a.dst);
+    const int N = a.N;
+    // one component of one cell from its NT source values (Madd<NT> order)
+    auto comb = [&](const float (&x)[NT]) {
+        if constexpr (NT == 3) {
+            return fa(fm(fac[0], x[0]), fa(fm(fac[1], x[1]), fm(fac[2], x[2])));
+        } else {
+            float acc = fm(fac[0], x[0]);
+#pragma unroll
+            for (int j = 1; j < NT; j++) acc = fa(acc, fm(fac[j], x[j]));
+            return acc;
+        }
+    };
+    auto finish = [&](float (&v)[3], float w) {
+        if (a.normalize) {
+            f3 r = normalize_vol(f3{v[0], v[1], v[2]}, w);
+            v[0] = r.x; v[1] = r.y; v[2] = r.z;
+        }
+    };
+    // Four cells per iteration with 16-byte loads and stores where every
+    // array allows it (N a multiple of 4, 16-byte aligned bases): four times
+    // the bytes in flight per thread; each cell's arithmetic is unchanged.
+    bool vec = (N & 3) == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0 &&
+               (!a.vol || (reinterpret_cast<uintptr_t>(a.vol) & 15) == 0);
+#pragma unroll
+    for (int j = 0; j < NT; j++) vec = vec && (reinterpret_cast<uintptr_t>(src[j]) & 15) == 0;
+    if (vec) {
+        const int N4 = N >> 2;
+        for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < N4; q += gridDim.x * blockDim.x) {
+            float v[4][3];
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                float4 x4[NT];
+#pragma unroll
+                for (int j = 0; j < NT; j++) x4[j] = reinterpret_cast<const float4*>(src[j] + (size_t)c * N)[q];
+#pragma unroll
+                for (int l = 0; l < 4; l++) {
+                    float x[NT];
+#pragma unroll
+                    for (int j = 0; j < NT; j++) x[j] = l == 0 ? x4[j].x : l == 1 ? x4[j].y : l == 2 ? x4[j].z : x4[j].w;
+                    v[l][c] = comb(x);
+                }
+            }
+            const float4 w4 = a.vol ? reinterpret_cast<const float4*>(a.vol)[q] : make_float4(1.f, 1.f, 1.f, 1.f);
+            finish(v[0], w4.x);
+            finish(v[1], w4.y);
+            finish(v[2], w4.z);
+            finish(v[3], w4.w);
+#pragma unroll
+            for (int c = 0; c < 3; c++)
+                reinterpret_cast<float4*>(dst + (size_t)c * N)[q] = make_float4(v[0][c], v[1][c], v[2][c], v[3][c]);
+        }
+        return;
+    }
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
+        float v[3];
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            float x[NT];
+#pragma unroll
+            for (int j = 0; j < NT; j++) x[j] = src[j][c * N + i];
+            v[c] = comb(x);
+        }
+        finish(v, a.vol ? a.vol[i] : 1.0f);
+        dst[i] = v[0]; dst[N + i] = v[1]; dst[2 * N + i] = v[2];
+    }
+}
+
+// ---------------------------------------------------------------- error norms
+struct ErrArgs {
+    DevCtl* ctl;
+    int N;
+    int nterm;
+    int slot[kMaxTerms];  // the last one's max norm is the torque of the new state (delM / k4 / dy)
+    TailArgs ta;          // constants, Heun, controller
+};
+
+// kErrTail as a kernel of its own, four cells a thread.
+template <int NT, bool HEUN, bool BAT>
+__global__ void __launch_bounds__(256) k_err_norms(ErrArgs a) {
+    DevCtl* ctl = a.ctl + (BAT ? blockIdx.y : 0);  // BAT: one grid row per instance
+    pdl_wait();
+    pdl_trigger();
+    if (!ctl->active) return;
+    const float* k[NT];
+    float e[NT];
+#pragma unroll
+    for (int j = 0; j < NT; j++) {
+        k[j] = ctl->k[a.slot[j]];
+        e[j] = a.ta.c[j];
+    }
+    const float* dm = ctl->k[a.slot[NT - 1]];
+    const int N = a.N;
+    float me = 0.f, md = 0.f, mr = 0.f;
+    int nan = 0;
+    // one component of the error estimate of one cell (Madd<NT> order)
+    auto comb = [&](const float (&x)[NT]) {
+        if constexpr (HEUN) {
+            return fs(x[0], x[1]);
+        } else if constexpr (NT == 3) {
+            return fa(fm(e[0], x[0]), fa(fm(e[1], x[1]), fm(e[2], x[2])));
+        } else {
+            float acc = fm(e[0], x[0]);
+#pragma unroll
+            for (int j = 1; j < NT; j++) acc = fa(acc, fm(e[j], x[j]));
+            return acc;
+        }
+    };
+    auto cell = [&](f3 E, f3 D) {
+        float e2 = dot3(E, E), d2 = dot3(D, D);
+        float en = __fsqrt_rn(e2), dn = __fsqrt_rn(d2);
+        float r = dn == 0.0f ? 0.0f : fd(en, dn);
+        nan |= (e2 != e2) | (d2 != d2);
+        me = fmaxf(me, e2);
+        md = fmaxf(md, d2);
+        mr = fmaxf(mr, r);
+    };
+    // four cells per iteration with 16-byte loads where every array allows
+    // it (the maxima do not depend on the order cells are visited in)
+    bool vec = (N & 3) == 0 && (reinterpret_cast<uintptr_t>(dm) & 15) == 0;
+#pragma unroll
+    for (int j = 0; j < NT; j++) vec = vec && (reinterpret_cast<uintptr_t>(k[j]) & 15) == 0;
+    if (vec) {
+        const int N4 = N >> 2;
+        for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < N4; q += gridDim.x * blockDim.x) {
+            float E[4][3], D[4][3];
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                float4 x4[NT];
+#pragma unroll
+                for (int j = 0; j < NT; j++) x4[j] = reinterpret_cast<const float4*>(k[j] + (size_t)c * N)[q];
+                const float4 d4 = reinterpret_cast<const float4*>(dm + (size_t)c * N)[q];
+                D[0][c] = d4.x; D[1][c] = d4.y; D[2][c] = d4.z; D[3][c] = d4.w;
+#pragma unroll
+                for (int l = 0; l < 4; l++) {
+                    float x[NT];
+#pragma unroll
+                    for (int j = 0; j < NT; j++) x[j] = l == 0 ? x4[j].x : l == 1 ? x4[j].y : l == 2 ? x4[j].z : x4[j].w;
+                    E[l][c] = comb(x);
+                }
+            }
+#pragma unroll
+            for (int l = 0; l < 4; l++) cell(f3{E[l][0], E[l][1], E[l][2]}, f3{D[l][0], D[l][1], D[l][2]});
+        }
+    } else {
+        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
+            float Ec[3];
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                float x[NT];
+#pragma unroll
+                for (int j = 0; j < NT; j++) x[j] = k[j][c * N + i];
+                Ec[c] = comb(x);
+            }
+            cell(f3{Ec[0], Ec[1], Ec[2]}, f3{dm[i], dm[N + i], dm[2 * N + i]});
+        }
+    }
+    err_finish(ErrMax{me, md, mr, nan}, true, a.ta, ctl, gridDim.x);
 }
 
 // ---------------------------------------------------------------- energies
@@ -766,7 +944,7 @@ struct SimImpl {
     int N;
     Mesh3 g;
     umag_demag* demag = nullptr;
-    float* bufs = nullptr;        // 2 + 7 slots of 3N
+    float* bufs = nullptr;        // 3 + 7 slots of 3N
     float* bd = nullptr;          // demag field 3N
     uint8_t* zero_regions = nullptr;
     float* dmi_pairs = nullptr;   // 7 x 32896 region-pair DMI coefficients
@@ -784,7 +962,7 @@ struct SimImpl {
     int launches_per_step = 0;
     double* esum = nullptr;            // energy term sums (kNE doubles)
     umag_tuning tune{{32, 8}, 256, 8, 4, 1};  // launch shapes (umag_sim_set_tuning)
-    TileMaps tmaps{};                          // TMA maps of the two magnetisation buffers
+    TileMaps tmaps{};                          // TMA maps of the three magnetisation buffers
     bool tile_ok = false;                      // the mesh and block shape allow tiles
     // batched ensemble class: nb same-size instances with uniform parameters
     int nb = 1;
@@ -796,204 +974,208 @@ struct SimImpl {
 // the ensemble class being captured
 static thread_local cudaStream_t g_launch_stream = nullptr;
 static cudaStream_t S() { return g_launch_stream ? g_launch_stream : ctx().stream; }
+// Kernels of one simulation overlap the next one's start (common.cuh); those
+// of an ensemble do not: waiting CTAs would hold the room that the other
+// classes' kernels, on streams of their own, can use.
+static bool overlap(const SimImpl* s) { return !s->batched && !g_launch_stream; }
 static unsigned ctl_grid(const SimImpl* s) { return (unsigned)((s->nb + 127) / 128); }
 
-// one torque evaluation of ctl->(m | mw) into ctl->k[slot] (or a direct buffer)
-static int launch_torque(SimImpl* s, int m_sel, int slot, float* tau_direct, float* beff, int* nl) {
+// the uniform-material instantiation: every term that it leaves out is off
+static bool uniform_terms(const SimImpl* s) {
+    const LocalArgs& la = s->la;
+    return s->zero_regions && !la.nodemag && !la.dbLUT && !la.cubic && !la.thermal && !la.frozen && la.precess &&
+           la.alpha_uniform && la.ms_uniform && (!la.anis || la.anis_uniform) && !la.openbc;
+}
+// Whether a step's stages and error estimate are formed in the torque kernel.
+// It saves their launches and the torque's way through memory; but the
+// kernel with maps and regions needs 64 registers for it, and holds fewer
+// warps.  us a step of RK45DP, separate / fused kernels: uniform material,
+// 256x256x4 258 / 253, 256x256x16 745 / 719, 512x512x32 6816 / 6747; region map
+// and per-cell maps, 256x256x4 299 / 287, 256x256x16 851 / 867, 512x512x32
+// 7771 / 8060.
+static bool fuse_tails(const SimImpl* s) {
+    if (!s->batched && s->tile_ok && s->tune.torque_tma && uniform_terms(s)) return true;
+    return (long)s->N * s->nb <= (1L << 19);
+}
+
+// one torque evaluation of magnetisation buffer m_sel into ctl->k[slot] (or a
+// direct buffer), and what follows it in the same kernel
+template <int TAIL>
+static cudaError_t torque_kernel(SimImpl* s, const LocalArgs& la, const TailArgs& ta, dim3 grd, dim3 blk, bool uni) {
+    const bool tile = s->zero_regions && s->tile_ok && s->tune.torque_tma;
+    auto k = s->batched ? k_local_torque<true, true, false, false, TAIL>
+             : tile && uni ? k_local_torque<true, false, true, true, TAIL>
+             : tile ? k_local_torque<true, false, true, false, TAIL>
+             : s->zero_regions ? k_local_torque<true, false, false, false, TAIL>
+                               : k_local_torque<false, false, false, false, TAIL>;
+    const size_t sm = !s->batched && tile ? tile_bytes(blk.x, blk.y, s->g.Nz) + 128 : 0;
+    return launch_pdl(overlap(s), k, grd, blk, sm, S(), la, s->tmaps, ta);
+}
+static int launch_torque(SimImpl* s, int m_sel, int slot, float* tau_direct, float* beff, int* nl,
+                         const TailArgs& ta = TailArgs{}) {
     if (s->p.enable_demag) {
         PassArgs a = s->pa;
-        a.m_sel = m_sel;
-        if (s->batched) UMAG_TRY(demag_launch_batch(s->demag, a, s->nb, S()));
-        else UMAG_TRY(demag_launch(s->demag, a, S()));
+        a.m_sel = m_sel != 0;
+        if (m_sel == 2) a.m_ind_w = &s->ctl->mw[1];
+        if (s->batched) UMAG_TRY(demag_launch_batch(s->demag, a, s->nb, S(), overlap(s)));
+        else UMAG_TRY(demag_launch(s->demag, a, S(), overlap(s)));
         if (nl) *nl += demag_launches(s->demag);
     }
     LocalArgs la = s->la;
     la.m_sel = m_sel;
+    la.early = s->p.enable_demag;
     la.out_slot = slot;
     la.tau_direct = tau_direct;
     la.beff = beff;
     const int bx = s->tune.torque_block[0], by = s->tune.torque_block[1];
     dim3 blk(bx, by, 1), grd((s->g.Nx + bx - 1) / bx, (s->g.Ny + by - 1) / by, s->g.Nz * s->nb);
-    // the uniform-material instantiation where every term it leaves out is off
-    const bool uni = s->zero_regions && !la.nodemag && !la.dbLUT && !la.cubic && !la.thermal && !beff &&
-                     !la.frozen && la.precess && la.alpha_uniform && la.ms_uniform && (!la.anis || la.anis_uniform) &&
-                     !la.openbc;
-    if (s->batched)
-        k_local_torque<true, true, false><<<grd, blk, 0, S()>>>(la, s->tmaps);
-    else if (s->zero_regions && s->tile_ok && s->tune.torque_tma && uni)
-        k_local_torque<true, false, true, true><<<grd, blk, tile_bytes(bx, by, s->g.Nz) + 128, S()>>>(la, s->tmaps);
-    else if (s->zero_regions && s->tile_ok && s->tune.torque_tma)
-        k_local_torque<true, false, true><<<grd, blk, tile_bytes(bx, by, s->g.Nz) + 128, S()>>>(la, s->tmaps);
-    else if (s->zero_regions)
-        k_local_torque<true, false, false><<<grd, blk, 0, S()>>>(la, s->tmaps);
-    else
-        k_local_torque<false, false, false><<<grd, blk, 0, S()>>>(la, s->tmaps);
-    UMAG_LAUNCH_CHECK();
+    const bool uni = uniform_terms(s) && !beff;
+    if (ta.kind == kStageTail) UMAG_CUDA(torque_kernel<kStageTail>(s, la, ta, grd, blk, uni));
+    else if (ta.kind == kErrTail) UMAG_CUDA(torque_kernel<kErrTail>(s, la, ta, grd, blk, uni));
+    else UMAG_CUDA(torque_kernel<kNoTail>(s, la, ta, grd, blk, uni));
     if (nl) *nl += 1;
     return UMAG_OK;
 }
 
-static int launch_stage(SimImpl* s, int src_m, std::initializer_list<int> slots, std::initializer_list<double> cs,
-                        bool scale_h, bool normalize, bool only_if_accepted, int* nl) {
+static int launch_stage(SimImpl* s, int src, int dst, std::initializer_list<int> slots,
+                        std::initializer_list<double> cs, bool normalize, bool begin, bool only_if_accepted, int* nl,
+                        int last_slot = -1) {
     StageArgs a{};
     a.ctl = s->ctl;
     a.N = s->N;
-    a.src_m = src_m;
-    a.nterm = 1 + (int)slots.size();
+    a.src = src;
+    a.dst = dst;
+    a.nterm = 1;
+    for (int sl : slots) a.slot[a.nterm++] = sl;
+    if (last_slot >= 0) a.slot[a.nterm++] = last_slot;
     int j = 1;
-    for (int sl : slots) a.slot[j++] = sl;
-    j = 1;
     for (double c : cs) a.c[j++] = (float)c;  // Go: untyped constant converted to float32
-    a.scale_h = scale_h;
     a.normalize = normalize;
+    a.begin = begin;
     a.only_if_accepted = only_if_accepted;
     a.vol = s->p.vol;
     const int th = s->tune.stage_threads;
     const dim3 g(s->batched ? (unsigned)((s->N + th - 1) / th) : (unsigned)grid_for(s->N, th, s->tune.stage_waves),
                  s->nb);
-#define STAGE(n)                                                    \
-    case n:                                                         \
-        if (s->batched) k_stage<n, true><<<g, th, 0, S()>>>(a);     \
-        else k_stage<n, false><<<g, th, 0, S()>>>(a);               \
-        break;
+    void (*k)(StageArgs) = nullptr;
     switch (a.nterm) {
-        STAGE(2) STAGE(3) STAGE(4) STAGE(5) STAGE(6)
+    case 2: k = s->batched ? k_stage<2, true> : k_stage<2, false>; break;
+    case 3: k = s->batched ? k_stage<3, true> : k_stage<3, false>; break;
+    case 4: k = s->batched ? k_stage<4, true> : k_stage<4, false>; break;
+    case 5: k = s->batched ? k_stage<5, true> : k_stage<5, false>; break;
+    case 6: k = s->batched ? k_stage<6, true> : k_stage<6, false>; break;
     default: return set_error(UMAG_E_ARG, "stage with %d terms", a.nterm);
     }
-#undef STAGE
-    UMAG_LAUNCH_CHECK();
+    UMAG_CUDA(launch_pdl(overlap(s), k, g, th, 0, S(), a));
     *nl += 1;
     return UMAG_OK;
 }
 
-static int launch_err(SimImpl* s, std::initializer_list<int> slots, std::initializer_list<double> es, int dm_slot,
-                      bool heun, int* nl) {
+// an evaluation into slot, then dst = normalize(m + h (sum_j cs_j k[slots_j] + cs_last k[slot]))
+static int torque_stage(SimImpl* s, int m_sel, int slot, int dst, std::initializer_list<int> slots,
+                        std::initializer_list<double> cs, int* nl, bool normalize = true) {
+    if (!fuse_tails(s)) {
+        UMAG_TRY(launch_torque(s, m_sel, slot, nullptr, nullptr, nl));
+        return launch_stage(s, 0, dst, slots, cs, normalize, false, false, nl, slot);
+    }
+    TailArgs t;
+    t.kind = kStageTail;
+    t.dst = dst;
+    t.normalize = normalize;
+    t.vol = s->p.vol;
+    for (int sl : slots) t.slot[t.nk++] = sl;
+    int j = 0;
+    for (double c : cs) t.c[j++] = (float)c;  // Go: untyped constant converted to float32
+    return launch_torque(s, m_sel, slot, nullptr, nullptr, nl, t);
+}
+// the step's last evaluation into slot, the error estimate
+// sum_j es_j k[slots_j] + es_last k[slot] and the controller
+static int torque_err(SimImpl* s, int m_sel, int slot, std::initializer_list<int> slots,
+                      std::initializer_list<double> es, bool heun, const CtlArgs& q, int* nl) {
+    TailArgs t;
+    t.kind = kErrTail;
+    t.heun = heun;
+    t.ctl = q;
+    for (int sl : slots) t.slot[t.nk++] = sl;
+    int j = 0;
+    for (double e : es) t.c[j++] = (float)e;
+    if (fuse_tails(s)) return launch_torque(s, m_sel, slot, nullptr, nullptr, nl, t);
+    UMAG_TRY(launch_torque(s, m_sel, slot, nullptr, nullptr, nl));
     ErrArgs a{};
     a.ctl = s->ctl;
     a.N = s->N;
-    a.nterm = (int)slots.size();
-    int j = 0;
-    for (int sl : slots) a.slot[j++] = sl;
-    j = 0;
-    for (double e : es) a.e[j++] = (float)e;
-    a.dm_slot = dm_slot;
-    a.heun = heun;
+    for (int sl : slots) a.slot[a.nterm++] = sl;
+    if (a.nterm == 0) a.slot[a.nterm++] = slot;  // Euler: the torque alone
+    a.slot[a.nterm++] = slot;
+    a.ta = t;
     const dim3 g(s->batched ? (unsigned)((s->N + 255) / 256) : (unsigned)grid_for(s->N, 256, s->tune.err_waves),
                  s->nb);
-#define ERRN(n, hn)                                                       \
-    do {                                                                  \
-        if (s->batched) k_err_norms<n, hn, true><<<g, 256, 0, S()>>>(a);  \
-        else k_err_norms<n, hn, false><<<g, 256, 0, S()>>>(a);            \
-    } while (0)
-    if (heun) ERRN(2, true);
-    else if (a.nterm == 2) ERRN(2, false);
-    else if (a.nterm == 4) ERRN(4, false);
-    else if (a.nterm == 6) ERRN(6, false);
+    void (*k)(ErrArgs) = nullptr;
+    if (heun) k = s->batched ? k_err_norms<2, true, true> : k_err_norms<2, true, false>;
+    else if (a.nterm == 2) k = s->batched ? k_err_norms<2, false, true> : k_err_norms<2, false, false>;
+    else if (a.nterm == 4) k = s->batched ? k_err_norms<4, false, true> : k_err_norms<4, false, false>;
+    else if (a.nterm == 6) k = s->batched ? k_err_norms<6, false, true> : k_err_norms<6, false, false>;
     else return set_error(UMAG_E_ARG, "error combination with %d terms", a.nterm);
-#undef ERRN
-    UMAG_LAUNCH_CHECK();
+    UMAG_CUDA(launch_pdl(overlap(s), k, g, 256, 0, S(), a));
     *nl += 1;
     return UMAG_OK;
 }
 
-// Slots: k[0] = k1 (FSAL), k[1..6] = k2..k7 buffers.
+// Slots: k[0] = k1 (FSAL), k[1..6] = k2..k7 buffers.  Each evaluation's kernel
+// writes the next stage's magnetisation to the working buffer that it does not
+// read (1 and 2 in turn).
 static int launch_step(SimImpl* s, int* nl) {
-    DevCtl* c = s->ctl;
-    k_step_begin<<<ctl_grid(s), 128, 0, S()>>>(c, s->nb);
-    UMAG_LAUNCH_CHECK();
-    *nl += 1;
+    auto begin = [&]() -> int {
+        UMAG_CUDA(launch_pdl(overlap(s), k_step_begin, ctl_grid(s), 128, 0, S(), s->ctl, s->nb));
+        *nl += 1;
+        return UMAG_OK;
+    };
     switch (s->sp.solver) {
     case 5: {  // engine/rk45dp.go:52-97
-        UMAG_TRY(launch_stage(s, 0, {0}, {1. / 5.}, true, true, false, nl));
-        UMAG_TRY(launch_torque(s, 1, 1, nullptr, nullptr, nl));
-        UMAG_TRY(launch_stage(s, 0, {0, 1}, {3. / 40., 9. / 40.}, true, true, false, nl));
-        UMAG_TRY(launch_torque(s, 1, 2, nullptr, nullptr, nl));
-        UMAG_TRY(launch_stage(s, 0, {0, 1, 2}, {44. / 45., -56. / 15., 32. / 9.}, true, true, false, nl));
-        UMAG_TRY(launch_torque(s, 1, 3, nullptr, nullptr, nl));
-        UMAG_TRY(launch_stage(s, 0, {0, 1, 2, 3}, {19372. / 6561., -25360. / 2187., 64448. / 6561., -212. / 729.},
-                              true, true, false, nl));
-        UMAG_TRY(launch_torque(s, 1, 4, nullptr, nullptr, nl));
-        UMAG_TRY(launch_stage(s, 0, {0, 1, 2, 3, 4},
-                              {9017. / 3168., -355. / 33., 46732. / 5247., 49. / 176., -5103. / 18656.}, true, true,
-                              false, nl));
-        UMAG_TRY(launch_torque(s, 1, 5, nullptr, nullptr, nl));
-        UMAG_TRY(launch_stage(s, 0, {0, 2, 3, 4, 5},
-                              {35. / 384., 500. / 1113., 125. / 192., -2187. / 6784., 11. / 84.}, true, true, false,
-                              nl));
-        UMAG_TRY(launch_torque(s, 1, 6, nullptr, nullptr, nl));
+        UMAG_TRY(launch_stage(s, 0, 1, {0}, {1. / 5.}, true, true, false, nl));
+        UMAG_TRY(torque_stage(s, 1, 1, 2, {0}, {3. / 40., 9. / 40.}, nl));
+        UMAG_TRY(torque_stage(s, 2, 2, 1, {0, 1}, {44. / 45., -56. / 15., 32. / 9.}, nl));
+        UMAG_TRY(torque_stage(s, 1, 3, 2, {0, 1, 2}, {19372. / 6561., -25360. / 2187., 64448. / 6561., -212. / 729.}, nl));
+        UMAG_TRY(torque_stage(s, 2, 4, 1, {0, 1, 2, 3},
+                              {9017. / 3168., -355. / 33., 46732. / 5247., 49. / 176., -5103. / 18656.}, nl));
+        UMAG_TRY(torque_stage(s, 1, 5, 2, {0, 2, 3, 4},
+                              {35. / 384., 500. / 1113., 125. / 192., -2187. / 6784., 11. / 84.}, nl));
         // rk45dp.go:95 weight differences, as exact rationals rounded to float32
-        UMAG_TRY(launch_err(s, {0, 2, 3, 4, 5, 6},
-                            {71. / 57600., -71. / 16695., 71. / 1920., -17253. / 339200., 22. / 525., -1. / 40.}, 6,
-                            false, nl));
-        k_controller<<<ctl_grid(s), 128, 0, S()>>>(c, s->nb, 0, 5, 6, 6, 0, 6);
-        break;
+        return torque_err(s, 2, 6, {0, 2, 3, 4, 5},
+                          {71. / 57600., -71. / 16695., 71. / 1920., -17253. / 339200., 22. / 525., -1. / 40.}, false,
+                          CtlArgs{0, 5, 6, 6, 0, 6, 2, 0}, nl);
     }
     case 3: {  // engine/rk23.go:58-83
-        UMAG_TRY(launch_stage(s, 0, {0}, {1. / 2.}, true, true, false, nl));
-        UMAG_TRY(launch_torque(s, 1, 1, nullptr, nullptr, nl));
-        UMAG_TRY(launch_stage(s, 0, {1}, {3. / 4.}, true, true, false, nl));
-        UMAG_TRY(launch_torque(s, 1, 2, nullptr, nullptr, nl));
-        UMAG_TRY(launch_stage(s, 0, {0, 1, 2}, {2. / 9., 1. / 3., 4. / 9.}, true, true, false, nl));
-        UMAG_TRY(launch_torque(s, 1, 3, nullptr, nullptr, nl));
-        UMAG_TRY(launch_err(s, {0, 1, 2, 3}, {5. / 72., -1. / 12., -1. / 9., 1. / 8.}, 3, false, nl));
-        k_controller<<<ctl_grid(s), 128, 0, S()>>>(c, s->nb, 0, 3, 4, 3, 0, 3);
-        break;
+        UMAG_TRY(launch_stage(s, 0, 1, {0}, {1. / 2.}, true, true, false, nl));
+        UMAG_TRY(torque_stage(s, 1, 1, 2, {}, {3. / 4.}, nl));
+        UMAG_TRY(torque_stage(s, 2, 2, 1, {0, 1}, {2. / 9., 1. / 3., 4. / 9.}, nl));
+        return torque_err(s, 1, 3, {0, 1, 2}, {5. / 72., -1. / 12., -1. / 9., 1. / 8.}, false,
+                          CtlArgs{0, 3, 4, 3, 0, 3, 1, 0}, nl);
     }
     case 2: {  // engine/heun.go:15-59
-        UMAG_TRY(launch_torque(s, 0, 0, nullptr, nullptr, nl));                      // dy0
-        UMAG_TRY(launch_stage(s, 0, {0}, {1.0}, true, false, false, nl));            // y = y + dt*dy0
-        UMAG_TRY(launch_torque(s, 1, 1, nullptr, nullptr, nl));                      // dy
-        UMAG_TRY(launch_err(s, {0, 1}, {1.0, -1.0}, 1, true, nl));                   // |dy0 - dy|
-        k_controller<<<ctl_grid(s), 128, 0, S()>>>(c, s->nb, 2, 2, 3, -1, -1, 2);
-        UMAG_LAUNCH_CHECK();
-        *nl += 1;
+        UMAG_TRY(begin());
+        UMAG_TRY(torque_stage(s, 0, 0, 1, {}, {1.0}, nl, false));  // dy0; y = y + dt*dy0
+        UMAG_TRY(torque_err(s, 1, 1, {0}, {}, true, CtlArgs{2, 2, 3, -1, -1, 2, 1, 0}, nl));  // dy; |dy0 - dy|
         // accepted: y = y + 0.5 dt dy - 0.5 dt dy0, normalised (heun.go:45-46)
-        UMAG_TRY(launch_stage(s, 1, {1, 0}, {0.5, -0.5}, true, true, true, nl));
-        k_step_end<<<ctl_grid(s), 128, 0, S()>>>(c, s->nb, 0);
-        UMAG_LAUNCH_CHECK();
-        *nl += 1;
-        return UMAG_OK;
+        return launch_stage(s, 0, 0, {1, 0}, {0.5, -0.5}, true, false, true, nl);
     }
     case 1: {  // engine/euler.go:11-36
-        UMAG_TRY(launch_torque(s, 0, 0, nullptr, nullptr, nl));           // dy0
-        UMAG_TRY(launch_err(s, {0, 0}, {1.0, -1.0}, 0, true, nl));        // max |dy0|
-        k_controller<<<ctl_grid(s), 128, 0, S()>>>(c, s->nb, 3, 1, 1, -1, -1, 1);
-        UMAG_LAUNCH_CHECK();
-        *nl += 1;
+        UMAG_TRY(begin());
+        UMAG_TRY(torque_err(s, 0, 0, {}, {}, true, CtlArgs{3, 1, 1, -1, -1, 1, 1, 0}, nl));  // dy0, max |dy0|
         // y = y + dt*dy0 (Madd2), normalised (euler.go:33-34)
-        UMAG_TRY(launch_stage(s, 0, {0}, {1.0}, true, true, true, nl));
-        k_step_end<<<ctl_grid(s), 128, 0, S()>>>(c, s->nb, 0);
-        UMAG_LAUNCH_CHECK();
-        *nl += 1;
-        return UMAG_OK;
+        return launch_stage(s, 1, 0, {0}, {1.0}, true, false, true, nl);
     }
     case 4: {  // engine/rk4.go:11-69
-        UMAG_TRY(launch_torque(s, 0, 0, nullptr, nullptr, nl));
-        UMAG_TRY(launch_stage(s, 0, {0}, {1. / 2.}, true, true, false, nl));
-        UMAG_TRY(launch_torque(s, 1, 1, nullptr, nullptr, nl));
-        UMAG_TRY(launch_stage(s, 0, {1}, {1. / 2.}, true, true, false, nl));
-        UMAG_TRY(launch_torque(s, 1, 2, nullptr, nullptr, nl));
-        UMAG_TRY(launch_stage(s, 0, {2}, {1.}, true, true, false, nl));
-        UMAG_TRY(launch_torque(s, 1, 3, nullptr, nullptr, nl));
-        UMAG_TRY(launch_err(s, {0, 3}, {1., -1.}, 3, false, nl));
-        k_controller<<<ctl_grid(s), 128, 0, S()>>>(c, s->nb, 1, 4, 5, -1, -1, 4);
-        UMAG_LAUNCH_CHECK();
-        *nl += 1;
-        UMAG_TRY(launch_stage(s, 0, {0, 1, 2, 3}, {1. / 6., 1. / 3., 1. / 3., 1. / 6.}, true, true, true, nl));
-        k_step_end<<<ctl_grid(s), 128, 0, S()>>>(c, s->nb, 1);
-        UMAG_LAUNCH_CHECK();
-        *nl += 1;
-        return UMAG_OK;
+        UMAG_TRY(begin());
+        UMAG_TRY(torque_stage(s, 0, 0, 1, {}, {1. / 2.}, nl));
+        UMAG_TRY(torque_stage(s, 1, 1, 2, {}, {1. / 2.}, nl));
+        UMAG_TRY(torque_stage(s, 2, 2, 1, {}, {1.}, nl));
+        UMAG_TRY(torque_err(s, 1, 3, {0}, {1., -1.}, false, CtlArgs{1, 4, 5, -1, -1, 4, 1, 1}, nl));
+        return launch_stage(s, 1, 0, {0, 1, 2, 3}, {1. / 6., 1. / 3., 1. / 3., 1. / 6.}, true, false, true, nl);
     }
     default:
         return set_error(UMAG_E_ARG, "unknown solver %d", s->sp.solver);
     }
-    UMAG_LAUNCH_CHECK();
-    *nl += 1;
-    k_step_end<<<ctl_grid(s), 128, 0, S()>>>(c, s->nb, 0);
-    UMAG_LAUNCH_CHECK();
-    *nl += 1;
-    return UMAG_OK;
 }
 
 static int sync_ctl_to_host(SimImpl* s) {
@@ -1086,7 +1268,7 @@ static void tile_setup(SimImpl* s) {
     const cuuint32_t box[4] = {(cuuint32_t)tile_pitch(bx), (cuuint32_t)tile_rows(by),
                                (cuuint32_t)(s->g.Nz > 1 ? 3 : 1), 3};
     const cuuint32_t es[4] = {1, 1, 1, 1};
-    for (int b = 0; b < 2; b++) {
+    for (int b = 0; b < 3; b++) {
         float* base = s->bufs + (size_t)b * 3 * s->N;
         if (reinterpret_cast<uintptr_t>(base) % 16 != 0) return;
         if (fn(&s->tmaps.map[b], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, dims, strides, box, es,
@@ -1173,8 +1355,8 @@ int sim_new(const umag_sim_params* p, const umag_solver_params* sp, umag_sim** o
     int st = UMAG_OK;
     size_t b3 = sizeof(float) * 3 * (size_t)s->N;
     auto fail = [&](int code) { sim_free(reinterpret_cast<umag_sim*>(s)); return code; };
-    if (cudaMalloc(&s->bufs, b3 * 9) != cudaSuccess) return fail(set_error(UMAG_E_NOMEM, "state buffers"));
-    if (cudaMemsetAsync(s->bufs, 0, b3 * 9, S()) != cudaSuccess) return fail(set_error(UMAG_E_CUDA, "state buffers"));
+    if (cudaMalloc(&s->bufs, b3 * 10) != cudaSuccess) return fail(set_error(UMAG_E_NOMEM, "state buffers"));
+    if (cudaMemsetAsync(s->bufs, 0, b3 * 10, S()) != cudaSuccess) return fail(set_error(UMAG_E_CUDA, "state buffers"));
     if (!p->regions) {
         if (cudaMalloc(&s->zero_regions, s->N) != cudaSuccess) return fail(set_error(UMAG_E_NOMEM, "regions"));
         if (cudaMemsetAsync(s->zero_regions, 0, s->N, S()) != cudaSuccess) return fail(set_error(UMAG_E_CUDA, "regions"));
@@ -1196,8 +1378,8 @@ int sim_new(const umag_sim_params* p, const umag_solver_params* sp, umag_sim** o
     DevCtl& c = *s->hctl;
     memset(&c, 0, sizeof(c));
     c.m = s->bufs;
-    c.mw = s->bufs + 3 * (size_t)s->N;
-    for (int i = 0; i < 7; i++) c.k[i] = s->bufs + (2 + i) * 3 * (size_t)s->N;
+    for (int i = 0; i < 2; i++) c.mw[i] = s->bufs + (1 + i) * 3 * (size_t)s->N;
+    for (int i = 0; i < 7; i++) c.k[i] = s->bufs + (3 + i) * 3 * (size_t)s->N;
     c.dt = sp->dt;
     c.alarm = 0.0;
     c.stop = INFINITY;
@@ -1215,7 +1397,7 @@ int sim_new(const umag_sim_params* p, const umag_solver_params* sp, umag_sim** o
     if (s->demag) {
         fill_pass_args(s->demag, s->pa);
         s->pa.m_ind = &s->ctl->m;
-        s->pa.m_ind_w = &s->ctl->mw;
+        s->pa.m_ind_w = &s->ctl->mw[0];
         s->pa.active = &s->ctl->active;
         s->pa.fault = &s->ctl->status;
         s->pa.vol = p->vol;
@@ -1239,7 +1421,7 @@ int sim_new(const umag_sim_params* p, const umag_solver_params* sp, umag_sim** o
     la.bd = s->bd;
     st = local_from_params(s);
     if (st != UMAG_OK) return fail(st);
-    la.mbuf1 = s->bufs + 3 * (size_t)s->N;
+    for (int i = 0; i < 2; i++) la.mbuf[i] = s->bufs + (1 + i) * 3 * (size_t)s->N;
     // default launch shapes for small meshes: enough CTAs to reach most SMs
     // (the autotuner may choose others; results do not depend on them)
     if ((long)((s->g.Nx + 31) / 32) * ((s->g.Ny + 7) / 8) * s->g.Nz < ctx().sm_count) s->tune.torque_block[1] = 2;
@@ -1851,8 +2033,8 @@ static int ens_class_new(EnsClass& C, const umag_ens_instance* in, const std::ve
     const size_t n3 = 3 * (size_t)s->N;
     UMAG_CUDA(cudaStreamCreateWithFlags(&C.st, cudaStreamNonBlocking));
     UMAG_CUDA(cudaEventCreateWithFlags(&C.done, cudaEventDisableTiming));
-    UMAG_CUDA(cudaMalloc(&s->bufs, sizeof(float) * n3 * 9 * nb));
-    UMAG_CUDA(cudaMemsetAsync(s->bufs, 0, sizeof(float) * n3 * 9 * nb, S()));
+    UMAG_CUDA(cudaMalloc(&s->bufs, sizeof(float) * n3 * 10 * nb));
+    UMAG_CUDA(cudaMemsetAsync(s->bufs, 0, sizeof(float) * n3 * 10 * nb, S()));
     UMAG_CUDA(cudaMalloc(&s->zero_regions, s->N));
     UMAG_CUDA(cudaMemsetAsync(s->zero_regions, 0, s->N, S()));
     s->p.regions = s->zero_regions;
@@ -1867,10 +2049,10 @@ static int ens_class_new(EnsClass& C, const umag_ens_instance* in, const std::ve
     memset(s->hctl, 0, sizeof(DevCtl) * nb);
     for (int b = 0; b < nb; b++) {
         DevCtl& c = s->hctl[b];
-        float* base = s->bufs + (size_t)b * 9 * n3;
+        float* base = s->bufs + (size_t)b * 10 * n3;
         c.m = base;
-        c.mw = base + n3;
-        for (int i = 0; i < 7; i++) c.k[i] = base + (2 + i) * n3;
+        for (int i = 0; i < 2; i++) c.mw[i] = base + (1 + i) * n3;
+        for (int i = 0; i < 7; i++) c.k[i] = base + (3 + i) * n3;
         c.bd = s->bd ? s->bd + (size_t)b * n3 : nullptr;
         c.dt = sp->dt;
         c.stop = INFINITY;
@@ -1947,7 +2129,7 @@ static int ens_class_new(EnsClass& C, const umag_ens_instance* in, const std::ve
         s->pa.spec = C.spec;
         s->pa.spec_stride = spec_elems;
         s->pa.m_ind = &s->ctl[0].m;
-        s->pa.m_ind_w = &s->ctl[0].mw;
+        s->pa.m_ind_w = &s->ctl[0].mw[0];
         s->pa.active = &s->ctl[0].active;
         s->pa.fault = &s->ctl[0].status;
         s->pa.ctl_stride = sizeof(DevCtl);

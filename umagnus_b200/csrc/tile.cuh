@@ -25,7 +25,7 @@ constexpr int kTileHaloX = 4;           // left halo rounded up to 16 bytes
 constexpr int kTileWaitLimit = 1 << 16;  // mbarrier polls before the error flag
 
 struct TileMaps {
-    CUtensorMap map[2];  // one per magnetisation buffer (state / working)
+    CUtensorMap map[3];  // one per magnetisation buffer (state / working)
 };
 
 __host__ __device__ constexpr int tile_pitch(int bx) { return bx + 2 * kTileHaloX; }
