@@ -133,6 +133,8 @@ __global__ void __launch_bounds__(256) k_adj_stage_fwd(AdjField a, StepFac f, in
                                                        const float* __restrict__ m, const float* k0,
                                                        const float* k1, const float* k2, float* mnext,
                                                        double* psum) {
+    pdl_wait();
+    pdl_trigger();
     const int N = a.N;
     double acc = 0;
     for (int I = blockIdx.x * blockDim.x + threadIdx.x; I < N; I += gridDim.x * blockDim.x) {
@@ -213,6 +215,8 @@ __global__ void __launch_bounds__(256) k_adj_rev_start(AdjField a, StepFac f, co
                                                        const float* __restrict__ m3, const float* __restrict__ B3,
                                                        const float* __restrict__ lam, float* lam2, float* gk0,
                                                        float* gk1, float* gk2, float* gm, float* wB) {
+    pdl_wait();
+    pdl_trigger();
     const int N = a.N;
     for (int I = blockIdx.x * blockDim.x + threadIdx.x; I < N; I += gridDim.x * blockDim.x) {
         float u[3];
@@ -247,6 +251,8 @@ __global__ void __launch_bounds__(256) k_adj_rev_start_heun(AdjField a, StepFac 
                                                             const float* __restrict__ B1,
                                                             const float* __restrict__ lam, float* lam2, float* gk0,
                                                             float* gm, float* wB) {
+    pdl_wait();
+    pdl_trigger();
     const int N = a.N;
     for (int I = blockIdx.x * blockDim.x + threadIdx.x; I < N; I += gridDim.x * blockDim.x) {
         float z[3];
@@ -288,6 +294,8 @@ __global__ void __launch_bounds__(256) k_adj_rev_stage(AdjField a, StepFac f, in
                                                        const float* __restrict__ mprev,
                                                        const float* __restrict__ Bprev, float* lam2, float* wBn,
                                                        float wprobe, double* acc) {
+    pdl_wait();
+    pdl_trigger();
     const int N = a.N;
     for (int I = blockIdx.x * blockDim.x + threadIdx.x; I < N; I += gridDim.x * blockDim.x) {
         const int ix = I % a.g.Nx, iy = (I / a.g.Nx) % a.g.Ny, iz = I / (a.g.Nx * a.g.Ny);
@@ -640,6 +648,8 @@ static StepFac step_fac(float h, bool heun) {
 }
 
 static unsigned gridN(const AdjImpl* s) { return (unsigned)grid_for(s->N, 256); }
+// a kernel of a step, overlapping the one before (common.cuh)
+#define ADJ_LAUNCH(k, ...) UMAG_CUDA(launch_pdl(true, k, gridN(s), 256, 0, AS(), __VA_ARGS__))
 
 // demag of v (3N) into out: Ms map and geometry (forward), or Ms = 1 and no
 // geometry (cotangent: the reverse kernel applies Ms and vol per cell)
@@ -651,7 +661,7 @@ static int adj_demag(AdjImpl* s, const float* v, const float* Ms, float* out) {
     a.Ms = Ms;
     a.Ms_mul = 1.0f;
     a.vol = Ms ? s->p.vol : nullptr;
-    return demag_launch(s->demag, a, AS());
+    return demag_launch(s->demag, a, AS(), true);
 }
 
 // one step m -> mout (engine/rk4.go:35-61 or engine/heun.go:27-43 with fixed
@@ -674,7 +684,7 @@ static int adj_step(AdjImpl* s, const AdjField& af, const StepFac& f, const floa
     const float* bd = s->demag ? s->w(W_BD) : nullptr;
     for (int q = 0; q < nst; q++) {
         UMAG_TRY(adj_demag(s, ms[q], s->Ms, s->w(W_BD)));
-        k_adj_stage_fwd<<<gridN(s), 256, 0, AS()>>>(af, f, q, ms[q], bd, Bs[q], k[q], m, k[0], nst > 1 ? k[1] : nullptr,
+        ADJ_LAUNCH(k_adj_stage_fwd, af, f, q, ms[q], bd, Bs[q], k[q], m, k[0], nst > 1 ? k[1] : nullptr,
                                                      nst > 2 ? k[2] : nullptr, next[q],
                                                      q == nst - 1 ? psum : nullptr);
         UMAG_LAUNCH_CHECK();
@@ -950,9 +960,9 @@ static int adj_rev_segment(AdjImpl* s, const AdjField& af, const StepFac& f, int
         // stage q's field cotangent lives in wb[q & 1] (the last stage: wb[1])
         const int nst = s->nst();
         if (s->heun)
-            k_adj_rev_start_heun<<<G, 256, 0, AS()>>>(af, f, ms[1], ks[0], ks[1], Bs[1], lam, lam2, gk[0], gm, wb[1]);
+            ADJ_LAUNCH(k_adj_rev_start_heun, af, f, ms[1], ks[0], ks[1], Bs[1], lam, lam2, gk[0], gm, wb[1]);
         else
-            k_adj_rev_start<<<G, 256, 0, AS()>>>(af, f, m, ks[0], ks[1], ks[2], ks[3], ms[3], Bs[3], lam, lam2,
+            ADJ_LAUNCH(k_adj_rev_start, af, f, m, ks[0], ks[1], ks[2], ks[3], ms[3], Bs[3], lam, lam2,
                                                   gk[0], gk[1], gk[2], gm, wb[1]);
         UMAG_LAUNCH_CHECK();
         for (int q = nst - 1; q >= 0; q--) {
@@ -960,7 +970,7 @@ static int adj_rev_segment(AdjImpl* s, const AdjField& af, const StepFac& f, int
             float* wnext = wb[(q + 1) & 1];
             UMAG_TRY(adj_demag(s, wcur, nullptr, s->w(W_BD)));
             const bool probe_prev = q == 0 && n - 1 >= p.avg_from && p.w_probe != 0;
-            k_adj_rev_stage<<<G, 256, 0, AS()>>>(af, f, q, s->A, ms[q], wcur, dw, gm, m, q > 0 ? ks[q - 1] : nullptr,
+            ADJ_LAUNCH(k_adj_rev_stage, af, f, q, s->A, ms[q], wcur, dw, gm, m, q > 0 ? ks[q - 1] : nullptr,
                                                   q > 0 ? gk[q - 1] : nullptr, q > 0 ? ms[q - 1] : nullptr,
                                                   q > 0 ? Bs[q - 1] : nullptr, lam2, wnext,
                                                   probe_prev ? wprobe : 0.f, s->acc);

@@ -89,6 +89,9 @@ struct PassArgs {
     float* const* m_ind;
     float* const* m_ind_w;
     int m_sel;
+    // the kernel before the first pass leaves the slots and the flag alone, so
+    // they can be read while it runs (later passes always can)
+    int early;
     int ncell;
     const int* active;
     const float* vol;

@@ -86,7 +86,7 @@ __device__ __forceinline__ void k_reg_a_body(const PassArgs& a, const int bx, co
 #pragma unroll
         for (int j = 0; j < 8; j++) {
             if (j < 4) {
-                const float2 p = __ldg(reinterpret_cast<const float2*>(mp + rowi + 2 * (t + TX * j)));
+                const float2 p = *reinterpret_cast<const float2*>(mp + rowi + 2 * (t + TX * j));
                 v[0][j] = make_float2(__fmul_rn(bsat, p.x), __fmul_rn(bsat, p.y));
             } else {
                 v[0][j] = make_float2(0.f, 0.f);
@@ -285,9 +285,10 @@ __device__ __forceinline__ void k_reg_c_body(const PassArgs& a, const int bx, co
     float2* twr = twz + S::TWZ;
     float2* Xs = twr + M;
     float2* ex = Xs + NZ * XP;
+    const bool off = inst_inactive(a, ib);
     pdl_wait();
     pdl_trigger();
-    if (inst_inactive(a, ib)) return;
+    if (off) return;
     const int tid = threadIdx.x;
     // the (y, component) slab of the spectrum by one bulk tensor copy into
     // the x/z scratch (Xs and the exchange lines, idle until the z phase has

@@ -8,11 +8,11 @@ namespace umag {
 static constexpr double kMu0f = 4 * 3.1415926535897932384626433 * 1e-7;  // clh/constants.clh:5
 
 // copypadmul2.cl:13-20: MU0*Ms (FP64 product rounded to float32) * vol * m
-__device__ __forceinline__ float scaled_m(const PassArgs& a, const float* __restrict__ m, int i, float msmul) {
+__device__ __forceinline__ float scaled_m(const PassArgs& a, const float* m, int i, float msmul) {
     float fac = a.Ms == nullptr ? msmul : __fmul_rn(msmul, __ldg(a.Ms + i));
     float bsat = (float)(kMu0f * (double)fac);
     float w = a.vol == nullptr ? 1.0f : __fmul_rn(1.0f, __ldg(a.vol + i));
-    return __fmul_rn(__fmul_rn(bsat, w), __ldg(m + i));
+    return __fmul_rn(__fmul_rn(bsat, w), m[i]);
 }
 
 // Per-instance views of PassArgs for batched launches (an ensemble of

@@ -60,10 +60,19 @@ __global__ void __launch_bounds__(4 * NPAR * Line<L>::T) k_x_fwd(const __grid_co
     const int c = blockIdx.y / a.Nz, z = blockIdx.y - c * a.Nz, y0 = blockIdx.x * 4, y = y0 + row, Nx = a.Nx;
     tw_copy(tw, a.fx.tw, M, tid, NT);
     tw_copy(twr, a.twr, S::WR, tid, NT);
+    const float* m = nullptr;
+    bool off = false;
+    if (a.early) {
+        m = inst_m(a, ib, c);
+        off = inst_inactive(a, ib);
+    }
     pdl_wait();
     pdl_trigger();
-    const float* m = inst_m(a, ib, c);  // (both reads in flight before the first use)
-    if (inst_inactive(a, ib)) {
+    if (!a.early) {
+        m = inst_m(a, ib, c);
+        off = inst_inactive(a, ib);
+    }
+    if (off) {
         cpa_wait_all();
         return;
     }
@@ -81,11 +90,11 @@ __global__ void __launch_bounds__(4 * NPAR * Line<L>::T) k_x_fwd(const __grid_co
         auto xof = [&](int i) { return 2 * (t + T * (i / LN::R1) + LN::B1 * (i % LN::R1)); };
         if (pairs) {
 #pragma unroll
-            for (int i = 0; i < NV; i++) f[i] = __ldg(reinterpret_cast<const float2*>(m + i0 + min(xof(i), Nx - 2)));
+            for (int i = 0; i < NV; i++) f[i] = *reinterpret_cast<const float2*>(m + i0 + min(xof(i), Nx - 2));
         } else {
 #pragma unroll
             for (int i = 0; i < NV; i++)
-                f[i] = make_float2(__ldg(m + i0 + min(xof(i), Nx - 1)), __ldg(m + i0 + min(xof(i) + 1, Nx - 1)));
+                f[i] = make_float2(m[i0 + min(xof(i), Nx - 1)], m[i0 + min(xof(i) + 1, Nx - 1)]);
         }
         if (uni) {
             const float bsat = (float)(kMu0f * (double)msm);  // scaled_m's rounding: (bsat * 1) * m = bsat * m
@@ -162,9 +171,10 @@ __global__ void __launch_bounds__(4 * NPAR * Line<L>::T) k_x_inv(const __grid_co
     const int c = blockIdx.y / a.Nz, z = blockIdx.y - c * a.Nz, y0 = blockIdx.x * 4, y = y0 + row, Nx = a.Nx;
     tw_copy(tw, a.fx.tw, M, tid, NT);
     tw_copy(twr, a.twr, S::WR, tid, NT);
+    const bool off = inst_inactive(a, ib);
     pdl_wait();
     pdl_trigger();
-    if (inst_inactive(a, ib)) {
+    if (off) {
         cpa_wait_all();
         return;
     }
@@ -245,9 +255,10 @@ template <int H, int N = 1> __device__ __forceinline__ void z_ramp(P2 (&u)[H]) {
 // 125 us inverse for the 605 MB (5.3 and 4.8 TB/s).
 template <int H, int NPAR> __global__ void __launch_bounds__(128) k_z_fwd(const __grid_constant__ PassArgs a) {
     const int ib = blockIdx.z;
+    const bool off = inst_inactive(a, ib);
     pdl_wait();
     pdl_trigger();
-    if (inst_inactive(a, ib)) return;
+    if (off) return;
     const long ps = (long)a.Ny * a.Lx, e = blockIdx.x * 128L + threadIdx.x;
     if (e >= ps) return;
     float2* col = inst_spec(a, ib) + (long)blockIdx.y * a.Pz * ps + e;
@@ -272,9 +283,10 @@ template <int H, int NPAR> __global__ void __launch_bounds__(128) k_z_fwd(const 
 }
 template <int H, int NPAR> __global__ void __launch_bounds__(128) k_z_inv(const __grid_constant__ PassArgs a) {
     const int ib = blockIdx.z;
+    const bool off = inst_inactive(a, ib);
     pdl_wait();
     pdl_trigger();
-    if (inst_inactive(a, ib)) return;
+    if (off) return;
     const long ps = (long)a.Ny * a.Lx, e = blockIdx.x * 128L + threadIdx.x;
     if (e >= ps) return;
     float2* col = inst_spec(a, ib) + (long)blockIdx.y * a.Pz * ps + e;
@@ -368,9 +380,10 @@ __global__ void __launch_bounds__(4 * NPAR * Line<L>::T, YShape<L, NPAR>::minb) 
         }
     }
     tw_copy(tw, a.fy.tw, P, tid, NT);
+    const bool off = inst_inactive(a, ib);
     pdl_wait();
     pdl_trigger();
-    if (inst_inactive(a, ib)) {  // (not before the copies in flight have landed)
+    if (off) {  // (not before the copies in flight have landed)
         cpa_wait_all();
         __syncthreads();
         for (int it = 0; a.Kblocked && it < 2 * kTileWaitLimit && !mbar_try_wait(&kbar, 0); it++) {}

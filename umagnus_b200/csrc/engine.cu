@@ -1012,10 +1012,11 @@ static cudaError_t torque_kernel(SimImpl* s, const LocalArgs& la, const TailArgs
     return launch_pdl(overlap(s), k, grd, blk, sm, S(), la, s->tmaps, ta);
 }
 static int launch_torque(SimImpl* s, int m_sel, int slot, float* tau_direct, float* beff, int* nl,
-                         const TailArgs& ta = TailArgs{}) {
+                         const TailArgs& ta = TailArgs{}, bool early = false) {
     if (s->p.enable_demag) {
         PassArgs a = s->pa;
         a.m_sel = m_sel != 0;
+        a.early = early;
         if (m_sel == 2) a.m_ind_w = &s->ctl->mw[1];
         if (s->batched) UMAG_TRY(demag_launch_batch(s->demag, a, s->nb, S(), overlap(s)));
         else UMAG_TRY(demag_launch(s->demag, a, S(), overlap(s)));
@@ -1071,11 +1072,15 @@ static int launch_stage(SimImpl* s, int src, int dst, std::initializer_list<int>
     return UMAG_OK;
 }
 
+// whether the kernel before an evaluation of a step leaves the controller record
+// alone: all but the first one's, which starts the step
+static bool later_eval(const SimImpl* s, int slot) { return slot != (s->sp.solver == 5 || s->sp.solver == 3 ? 1 : 0); }
+
 // an evaluation into slot, then dst = normalize(m + h (sum_j cs_j k[slots_j] + cs_last k[slot]))
 static int torque_stage(SimImpl* s, int m_sel, int slot, int dst, std::initializer_list<int> slots,
                         std::initializer_list<double> cs, int* nl, bool normalize = true) {
     if (!fuse_tails(s)) {
-        UMAG_TRY(launch_torque(s, m_sel, slot, nullptr, nullptr, nl));
+        UMAG_TRY(launch_torque(s, m_sel, slot, nullptr, nullptr, nl, TailArgs{}, later_eval(s, slot)));
         return launch_stage(s, 0, dst, slots, cs, normalize, false, false, nl, slot);
     }
     TailArgs t;
@@ -1086,7 +1091,7 @@ static int torque_stage(SimImpl* s, int m_sel, int slot, int dst, std::initializ
     for (int sl : slots) t.slot[t.nk++] = sl;
     int j = 0;
     for (double c : cs) t.c[j++] = (float)c;  // Go: untyped constant converted to float32
-    return launch_torque(s, m_sel, slot, nullptr, nullptr, nl, t);
+    return launch_torque(s, m_sel, slot, nullptr, nullptr, nl, t, later_eval(s, slot));
 }
 // the step's last evaluation into slot, the error estimate
 // sum_j es_j k[slots_j] + es_last k[slot] and the controller
@@ -1099,8 +1104,8 @@ static int torque_err(SimImpl* s, int m_sel, int slot, std::initializer_list<int
     for (int sl : slots) t.slot[t.nk++] = sl;
     int j = 0;
     for (double e : es) t.c[j++] = (float)e;
-    if (fuse_tails(s)) return launch_torque(s, m_sel, slot, nullptr, nullptr, nl, t);
-    UMAG_TRY(launch_torque(s, m_sel, slot, nullptr, nullptr, nl));
+    if (fuse_tails(s)) return launch_torque(s, m_sel, slot, nullptr, nullptr, nl, t, later_eval(s, slot));
+    UMAG_TRY(launch_torque(s, m_sel, slot, nullptr, nullptr, nl, TailArgs{}, later_eval(s, slot)));
     ErrArgs a{};
     a.ctl = s->ctl;
     a.N = s->N;
