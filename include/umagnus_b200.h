@@ -306,7 +306,7 @@ int umag_sim_torque(umag_sim* s, float* tx, float* ty, float* tz, float* bx, flo
 int umag_sim_steps(umag_sim* s, int n);
 /* engine/run.go:190 Run(seconds): steps until the simulated time reaches
  * t+seconds (alarm honoured by adaptDt, engine/run.go:181-184), checking
- * the device time every `chunk` steps; max_steps bounds the loop. */
+ * the device time at least every `chunk` steps; max_steps bounds the loop. */
 int umag_sim_run(umag_sim* s, double seconds, int chunk, long long max_steps);
 int umag_sim_get_state(umag_sim* s, umag_solver_state* st);
 int umag_sim_set_time(umag_sim* s, double time, double dt);
@@ -415,9 +415,9 @@ int umag_ens_set_m(umag_ens* e, int i, const float* host_m);
 int umag_ens_get_m(umag_ens* e, int i, float* host_m);
 int umag_ens_get_state(umag_ens* e, int i, umag_solver_state* st);
 /* engine/run.go:190 Run(seconds) for every instance from its own current
- * time.  Each class (instances of one mesh) replays its own CUDA graph of 16
- * steps on its own stream, fed and checked by the host every `chunk`
- * replays independently of the other classes (at most max_replays replays
+ * time.  Each class (instances of one mesh) replays its own CUDA graphs on its
+ * own stream, fed and checked by the host at least every
+ * `chunk` * 16 steps independently of the other classes (at most max_replays * 16
  * per class); finished instances leave their class's batch (compaction) and
  * return at the next run.  No counterpart in the reference. */
 int umag_ens_run(umag_ens* e, double seconds, int chunk, long long max_replays);

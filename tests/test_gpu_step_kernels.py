@@ -5,6 +5,9 @@ Both forms of the step are covered: small meshes form the next stage (and the
 error estimate) inside the torque kernel, large ones in kernels of their own.
 Every operation is rounded the same way in all of them, so the results are
 equal bit for bit.
+
+And what run() queues ahead of what it knows changes nothing, nor does the
+compaction of an ensemble's batch.
 """
 import numpy as np
 import pytest
@@ -106,3 +109,59 @@ def test_step_equals_device_ops(solver, N, regions, geom):
     assert torch.equal(sim.get_m(), want2)
     sim.free()
     probe.free()
+
+
+@pytest.mark.parametrize("chunk", [1, 3, 16, 64, 1000])
+def test_run_does_not_depend_on_the_block_size(chunk):
+    """run() queues steps ahead of what it knows; steps past the stop time change nothing."""
+    from umagnus_b200 import engine
+
+    def start():
+        s = engine.Simulation((40, 24, 1), (4e-9, 4e-9, 3e-9), 8e5, 1.3e-11, 0.1, B_ext=(0, 0, 0.01))
+        s.set_m(torch.randn((3, 1, 24, 40), device="cuda", generator=torch.Generator("cuda").manual_seed(9)))
+        return s
+
+    a, b = start(), start()
+    T = 8e-12
+    a.run(T, chunk=chunk)
+    b.run(T)
+    assert a.state() == b.state() and a.state()["status"] == 0
+    assert a.state()["time"] >= T * (1 - 1e-12)
+    assert torch.equal(a.get_m(), b.get_m())
+    # bounded: exactly max_steps attempts
+    c = start()
+    c.run(1.0, chunk=chunk, max_steps=21)
+    st = c.state()
+    assert st["nsteps"] + st["nundone"] == 21
+    d = start()
+    d.steps(21)
+    assert torch.equal(c.get_m(), d.get_m())
+    a.run(T, chunk=chunk)  # a second run restarts from the stop time
+    assert a.state()["time"] >= 2 * T * (1 - 1e-12)
+    for s in (a, b, c, d):
+        s.free()
+
+
+def test_ensemble_compacts_long_runs():
+    """Stiff instances among soft ones run several hundred steps longer, enough for a smaller batch: all still
+    equal their single runs."""
+    from umagnus_b200 import engine
+    insts = [dict(N=(32, 32, 1), cell=(4e-9, 4e-9, 3e-9), Msat=8e5, Aex=2e-11 if i in (1, 6) else 2e-12, alpha=0.1,
+                  B_ext=(0.0, 0.0, 0.01 * i)) for i in range(9)]
+    rng = np.random.default_rng(4)
+    m0 = [rng.standard_normal((3, 1, 32, 32)).astype(np.float32) for _ in insts]
+    T = 1e-10
+    ens = engine.Ensemble(insts)
+    for i, m in enumerate(m0):
+        ens.set_m(i, m)
+    ens.run(T)
+    n = [ens.state(i)["nsteps"] for i in range(9)]
+    assert max(n) - sorted(n)[6] > 128, n  # seven finish while the others have far to go
+    for i, d in enumerate(insts):
+        sim = engine.Simulation(d["N"], d["cell"], d["Msat"], d["Aex"], d["alpha"], B_ext=d["B_ext"])
+        sim.set_m(m0[i])
+        sim.run(T)
+        assert ens.state(i) == sim.state()
+        assert np.array_equal(np.asarray(ens.get_m(i)), sim.get_m().cpu().numpy()), i
+        sim.free()
+    ens.free()

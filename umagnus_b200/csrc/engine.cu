@@ -10,9 +10,11 @@
 // through a device-side slot table: accepting a step swaps the state and
 // working magnetisation slots and moves k7 into the k1 slot (FSAL,
 // engine/stepcontroller.go:76-78) without copying.
+#include <algorithm>
 #include <cmath>
 #include <cstddef>
 #include <cstring>
+#include <map>
 #include <thread>
 #include <vector>
 
@@ -952,6 +954,9 @@ struct SimImpl {
     LocalConsts* kc_dev = nullptr;
     DevCtl* ctl = nullptr;        // device
     DevCtl* hctl = nullptr;       // pinned host mirror
+    // run(): the controller records after the blocks of steps in flight
+    DevCtl* hpoll = nullptr;      // pinned, 2
+    cudaEvent_t polled[2] = {nullptr, nullptr};
     PassArgs pa{};
     LocalArgs la{};
     bool need_k1 = true;
@@ -1380,6 +1385,10 @@ int sim_new(const umag_sim_params* p, const umag_solver_params* sp, umag_sim** o
     }
     if (cudaMalloc(&s->ctl, sizeof(DevCtl)) != cudaSuccess) return fail(set_error(UMAG_E_NOMEM, "ctl"));
     if (cudaMallocHost(&s->hctl, sizeof(DevCtl)) != cudaSuccess) return fail(set_error(UMAG_E_NOMEM, "ctl host"));
+    if (cudaMallocHost(&s->hpoll, 2 * sizeof(DevCtl)) != cudaSuccess) return fail(set_error(UMAG_E_NOMEM, "ctl host"));
+    for (auto& e : s->polled)
+        if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess)
+            return fail(set_error(UMAG_E_CUDA, "poll events"));
     DevCtl& c = *s->hctl;
     memset(&c, 0, sizeof(c));
     c.m = s->bufs;
@@ -1475,6 +1484,9 @@ int sim_free(umag_sim* h) {
     cudaFree(s->esum);
     cudaFree(s->ctl);
     if (s->hctl) cudaFreeHost(s->hctl);
+    if (s->hpoll) cudaFreeHost(s->hpoll);
+    for (auto e : s->polled)
+        if (e) cudaEventDestroy(e);
     delete s;
     return UMAG_OK;
 }
@@ -1539,6 +1551,18 @@ int sim_steps(umag_sim* h, int n) {
     return run_steps(s, n);
 }
 
+// Steps from record c to its stop time, if the time step stayed as it is.
+static long long steps_left(const DevCtl& c) {
+    if (!(c.t < c.stop) || c.status != 0) return 0;
+    const double n = std::ceil((c.stop - c.t) / c.dt);
+    return n >= 1 ? (n < 1e9 ? (long long)n : 1000000000LL) : 1;
+}
+
+// Steps queued past the stop time do nothing but cost their launches (a tenth
+// of the run for 27 steps of 256x256x16 queued as 64), and waiting for each
+// step would leave gaps.  So blocks of steps are queued as far as the last
+// record says that they are needed, two blocks ahead at most: first 8 steps
+// (the time step still grows), then 16.
 int sim_run(umag_sim* h, double seconds, int chunk, long long max_steps) {
     SimImpl* s = reinterpret_cast<SimImpl*>(h);
     UMAG_REQUIRE(s && seconds >= 0, "bad argument");
@@ -1549,17 +1573,31 @@ int sim_run(umag_sim* h, double seconds, int chunk, long long max_steps) {
     s->hctl->alarm = stop;  // engine/run.go:190-195: adaptDt must not cross it
     UMAG_TRY(push_ctl(s));
     s->need_k1 = true;      // RunWhile frees the stepper (engine/run.go:207)
-    long long done = 0;
-    while (done < max_steps) {
-        long long n = chunk;
-        if (max_steps - done < n) n = max_steps - done;
-        UMAG_TRY(run_steps(s, n));
-        done += n;
-        UMAG_TRY(sync_ctl_to_host(s));
-        if (s->hctl->status != 0) return set_error(UMAG_E_SOLVER, "solver failure code %d at t=%g", s->hctl->status,
-                                                   s->hctl->t);
-        if (!(s->hctl->t < stop)) break;
+    if (max_steps > 0) UMAG_TRY(ensure_k1(s));
+    long long queued = 0, known = 0, ends[2] = {0, 0}, left = steps_left(*s->hctl);
+    int in_flight = 0, oldest = 0;
+    while (left > 0) {
+        long long n = std::min(left - (queued - known), max_steps - queued);
+        if (n > 0 && in_flight < 2) {
+            n = std::min(n, (long long)std::min(chunk, known > 0 && n >= 32 ? 16 : 8));
+            UMAG_TRY(run_steps(s, n));
+            queued += n;
+            const int q = (oldest + in_flight++) % 2;
+            ends[q] = queued;
+            UMAG_CUDA(cudaMemcpyAsync(s->hpoll + q, s->ctl, sizeof(DevCtl), cudaMemcpyDeviceToHost, S()));
+            UMAG_CUDA(cudaEventRecord(s->polled[q], S()));
+            continue;
+        }
+        if (in_flight == 0) break;  // max_steps
+        UMAG_CUDA(cudaEventSynchronize(s->polled[oldest]));
+        left = steps_left(s->hpoll[oldest]);
+        known = ends[oldest];
+        oldest ^= 1;
+        in_flight--;
     }
+    UMAG_TRY(sync_ctl_to_host(s));
+    if (s->hctl->status != 0) return set_error(UMAG_E_SOLVER, "solver failure code %d at t=%g", s->hctl->status,
+                                               s->hctl->t);
     return UMAG_OK;
 }
 
@@ -1952,6 +1990,10 @@ int sim_set_param(umag_sim* h, int which, const float* values, float mul) {
 // state buffers stay where they are, the records point at them) and the
 // class's graph is recaptured for the smaller batch, so finished instances
 // stop costing launches.  Every instance's arithmetic is unchanged.
+constexpr int kEnsUnit = 4;        // steps of one graph of a class
+constexpr int kEnsReplay = 16;     // steps that `chunk` and `max_replays` count in
+constexpr size_t kEnsGraphs = 12;  // graphs a class keeps
+constexpr int kEnsCompact = 64;    // steps that must be left for a new batch size to pay
 struct EnsClass {
     SimImpl* s = nullptr;
     // a general instance: one simulation made by sim_new from a full
@@ -1965,21 +2007,22 @@ struct EnsClass {
     int n_all = 0;             // instances of the class; the first s->nb slots are in the batch
     cudaStream_t st = nullptr;
     cudaEvent_t done = nullptr;
-    cudaGraphExec_t gexec = nullptr;  // graph_steps steps of the current batch
-    int gexec_nb = 0;                 // the batch size gexec was captured for
+    std::map<int, cudaGraphExec_t> graphs;  // kEnsUnit steps, by batch size
     bool busy = false, finished = false;
-    long long replays = 0;
+    long long units = 0;  // queued in this run
 };
 struct EnsImpl {
     std::vector<EnsClass> cls;
     std::vector<std::pair<int, int>> where;  // instance -> (class, slot in class)
     umag_solver_params sp;
-    int graph_steps = 16;
 };
 
+static void ens_drop_graphs(EnsClass& c) {
+    for (auto& g : c.graphs) cudaGraphExecDestroy(g.second);
+    c.graphs.clear();
+}
 static void ens_class_free(EnsClass& c) {
-    if (c.gexec) cudaGraphExecDestroy(c.gexec);
-    c.gexec = nullptr;
+    ens_drop_graphs(c);
     if (c.s && c.general) {
         sim_free(reinterpret_cast<umag_sim*>(c.s));
         c.s = nullptr;
@@ -2274,14 +2317,16 @@ int ens_get_state(umag_ens* h, int i, umag_solver_state* st) {
     return UMAG_OK;
 }
 
-// graph_steps steps of class C's current batch, captured on its stream
-static int ens_capture(EnsImpl* e, EnsClass& C) {
-    if (C.gexec && C.gexec_nb == C.s->nb) return UMAG_OK;  // still valid (shapes unchanged)
-    if (C.gexec) { cudaGraphExecDestroy(C.gexec); C.gexec = nullptr; }
+// kEnsUnit steps of class C's current batch, captured on its stream (which is
+// idle).  A batch size comes back in every run, so its graph is kept.
+static int ens_capture(EnsClass& C) {
+    if (C.graphs.count(C.s->nb)) return UMAG_OK;
+    if (C.graphs.size() >= kEnsGraphs) ens_drop_graphs(C);
+    cudaGraphExec_t g = nullptr;
     g_launch_stream = C.st;
-    const int st = capture_steps(C.s, e->graph_steps, &C.gexec);
+    const int st = capture_steps(C.s, kEnsUnit, &g);
     g_launch_stream = nullptr;
-    C.gexec_nb = st == UMAG_OK ? C.s->nb : 0;
+    if (st == UMAG_OK) C.graphs[C.s->nb] = g;
     return st;
 }
 
@@ -2300,6 +2345,13 @@ static int ens_compact(EnsImpl* e, int ci) {
         if (s->hctl[b].t < s->hctl[b].stop && s->hctl[b].status == 0) order.push_back(b);
     const int na = (int)order.size();
     if (na == 0 || 4 * na > 3 * nb) return UMAG_OK;
+    // A smaller batch needs a graph of its own, about a millisecond of this
+    // thread for 100 launches; what a finished instance costs is the early exit
+    // of its CTAs.  (48 films of up to 134 steps: 34.9 ms
+    // compacting at every poll, 21.6 ms without.)
+    long long left = 0;
+    for (int b = 0; b < nb; b++) left = std::max(left, steps_left(s->hctl[b]));
+    if (left < kEnsCompact && !C.graphs.count(na)) return UMAG_OK;
     for (int b = 0; b < nb; b++)
         if (!(s->hctl[b].t < s->hctl[b].stop && s->hctl[b].status == 0)) order.push_back(b);
     std::vector<DevCtl> ctl(nb);
@@ -2328,16 +2380,20 @@ static int ens_compact(EnsImpl* e, int ci) {
     UMAG_CUDA(cudaMemcpyAsync(C.params, hp.data(), sizeof(float) * hp.size(), cudaMemcpyHostToDevice, S()));
     UMAG_TRY(ens_push_all(C));
     s->nb = na;
-    return ens_capture(e, C);
+    return ens_capture(C);
 }
 
 // engine/run.go:190 Run(seconds) for every instance: each runs until its own
 // time reaches start + seconds (its dt honours that alarm).  Classes advance
-// independently, `chunk` graph replays at a time (at most max_replays each).
+// independently, at most `chunk` * kEnsReplay steps at a time (and max_replays *
+// kEnsReplay in all).  A block covers three quarters of what its slowest instance
+// needs by its last time step (first 8 steps, while the time step still
+// grows): steps past the stop time do nothing but cost their launches.
 int ens_run(umag_ens* h, double seconds, int chunk, long long max_replays) {
     EnsImpl* e = reinterpret_cast<EnsImpl*>(h);
     UMAG_REQUIRE(e && seconds >= 0, "bad argument");
     if (chunk <= 0) chunk = 8;
+    const long long per = kEnsReplay / kEnsUnit, max_units = max_replays > (1LL << 60) ? 1LL << 62 : max_replays * per;
     for (auto& C : e->cls) {
         SimImpl* s = C.s;
         UMAG_TRY(ens_sync_all(C));
@@ -2349,10 +2405,10 @@ int ens_run(umag_ens* h, double seconds, int chunk, long long max_replays) {
         UMAG_TRY(ens_push_all(C));
         s->need_k1 = true;  // RunWhile frees the stepper (engine/run.go:207)
         UMAG_TRY(ensure_k1(s));
-        UMAG_TRY(ens_capture(e, C));
+        UMAG_TRY(ens_capture(C));
         C.busy = false;
         C.finished = false;
-        C.replays = 0;
+        C.units = 0;
     }
     UMAG_CUDA(cudaDeviceSynchronize());
     for (;;) {
@@ -2376,15 +2432,19 @@ int ens_run(umag_ens* h, double seconds, int chunk, long long max_replays) {
                                          d.status, d.t);
                     running += d.t < d.stop;
                 }
-                if (running == 0 || C.replays >= max_replays) {
+                if (running == 0 || C.units >= max_units) {
                     C.finished = true;
                     continue;
                 }
                 UMAG_TRY(ens_compact(e, (int)ci));
             }
-            // the next chunk, then the batch's records back to the host
-            for (int k = 0; k < chunk && C.replays < max_replays; k++, C.replays++)
-                UMAG_CUDA(cudaGraphLaunch(C.gexec, C.st));
+            // the next block, then the batch's records back to the host
+            long long last = 0;
+            for (int b = 0; b < s->nb; b++) last = std::max(last, steps_left(s->hctl[b]));
+            const long long steps = C.units == 0 ? 8 : std::max((3 * last + 3) / 4, std::min(last, 8LL));
+            const long long want = (steps + kEnsUnit - 1) / kEnsUnit;
+            for (long long k = std::min(want, chunk * per); k > 0 && C.units < max_units; k--, C.units++)
+                UMAG_CUDA(cudaGraphLaunch(C.graphs[s->nb], C.st));
             UMAG_CUDA(cudaMemcpyAsync(s->hctl, s->ctl, sizeof(DevCtl) * s->nb, cudaMemcpyDeviceToHost, C.st));
             UMAG_CUDA(cudaEventRecord(C.done, C.st));
             C.busy = true;
@@ -2438,7 +2498,7 @@ int ens_set_tuning(umag_ens* h, int cls, const umag_tuning* t) {
     UMAG_REQUIRE(cls >= 0 && cls < (int)e->cls.size(), "class %d out of range", cls);
     EnsClass& C = e->cls[cls];
     UMAG_TRY(sim_set_tuning(reinterpret_cast<umag_sim*>(C.s), t));
-    if (C.gexec) { cudaGraphExecDestroy(C.gexec); C.gexec = nullptr; }
+    ens_drop_graphs(C);
     return UMAG_OK;
 }
 
