@@ -38,7 +38,12 @@ template <int L, int NPAR> struct XShape {
     static constexpr int SR = NPAR * SP + (T < 8 ? 4 : 0);       // rows
     static constexpr int ZP = pitch16(M + 1, 4);                  // half-spectrum rows
     static constexpr int WR = M / 2 + 1;                          // exp(-2 pi i k / 2M), k <= M/2
-    static constexpr size_t smem = sizeof(float2) * ((size_t)M + WR + 4 * SR + 4 * ZP);
+    // the rows and the exchange lines share their room
+    static constexpr size_t smem = sizeof(float2) * ((size_t)M + WR + 4 * (SR > ZP ? SR : ZP));
+    // forward: values, scales and addresses
+    static constexpr int regs = (LN::NE <= 8 ? 64 : LN::NE <= 12 ? 80 : 96) + (NPAR == 1 ? 32 : 0);
+    static constexpr int minb0 = 65536 / (regs * ((NT + 31) / 32 * 32)), minb1 = (int)(227 * 1024 / (smem + 1024));
+    static constexpr int minb = minb0 < minb1 ? (minb0 < 16 ? minb0 : 16) : (minb1 < 16 ? minb1 : 16);
 };
 
 // Forward: z[n] = x[2n] + i x[2n+1] of every row (zero above Nx), transform of
@@ -47,14 +52,17 @@ template <int L, int NPAR> struct XShape {
 // meshes.  Up to some 100,000 cells the time is the latency of one CTA (the
 // controller read, the rows, one exchange, the unpack), above it the spectrum
 // stores.  64x64: 3.1 us, 250x250 with a geometry map: 5.0 us (the
-// runtime-planned pass took 45.7), 1024x1024: 25.1 us (30.6).
+// runtime-planned pass took 45.7), 1024x1024: 25.1 us (30.6).  Large meshes with
+// an Ms map are bound by latency at the CTAs that fit: with rows and exchange
+// lines in one room, a register cap, and each parity scaling half of the values that both
+// need, RK45DP on 512x512x32 with regions takes 7479 us a step (7771 before).
 template <int L, int NPAR>
-__global__ void __launch_bounds__(4 * NPAR * Line<L>::T) k_x_fwd(const __grid_constant__ PassArgs a) {
+__global__ void __launch_bounds__(4 * NPAR * Line<L>::T, XShape<L, NPAR>::minb) k_x_fwd(const __grid_constant__ PassArgs a) {
     using S = XShape<L, NPAR>;
     using LN = typename S::LN;
     constexpr int M = S::M, T = S::T, NT = S::NT;
     extern __shared__ __align__(16) float2 sm[];
-    float2 *tw = sm, *twr = tw + M, *ex = twr + S::WR, *Zs = ex + 4 * S::SR;
+    float2 *tw = sm, *twr = tw + M, *ex = twr + S::WR, *Zs = ex;
     const int ib = blockIdx.z;
     const int tid = threadIdx.x, p = tid % NPAR, t = (tid / NPAR) % T, row = tid / (NPAR * T);
     const int c = blockIdx.y / a.Nz, z = blockIdx.y - c * a.Nz, y0 = blockIdx.x * 4, y = y0 + row, Nx = a.Nx;
@@ -101,26 +109,42 @@ __global__ void __launch_bounds__(4 * NPAR * Line<L>::T) k_x_fwd(const __grid_co
 #pragma unroll
             for (int i = 0; i < NV; i++) f[i] = make_float2(__fmul_rn(bsat, f[i].x), __fmul_rn(bsat, f[i].y));
         } else {
-            float2 bs[NV];
+            // the two parities of a row need the same values: each scales half of them
+            constexpr int NS = (NV + NPAR - 1) / NPAR;
+            float2 bs[NS], g[NS];
+            int x0[NS], x1[NS];
 #pragma unroll
-            for (int i = 0; i < NV; i++) {
-                const int x0 = i0 + min(xof(i), Nx - 1), x1 = i0 + min(xof(i) + 1, Nx - 1);
-                bs[i] = a.Ms ? make_float2(__ldg(a.Ms + x0), __ldg(a.Ms + x1)) : make_float2(1.f, 1.f);
+            for (int i = 0; i < NS; i++) {
+                const bool odd = NPAR == 2 && p && 2 * i + 1 < NV;
+                const int x = odd ? xof(NPAR * i + 1) : xof(NPAR * i);
+                x0[i] = i0 + min(x, Nx - 1);
+                x1[i] = i0 + min(x + 1, Nx - 1);
+                g[i] = odd ? f[NPAR * i + 1 < NV ? NPAR * i + 1 : 0] : f[NPAR * i];
+                bs[i] = a.Ms ? make_float2(__ldg(a.Ms + x0[i]), __ldg(a.Ms + x1[i])) : make_float2(1.f, 1.f);
             }
 #pragma unroll
-            for (int i = 0; i < NV; i++)  // MU0*Ms: FP64 product rounded to float32 (copypadmul2.cl:13-20)
+            for (int i = 0; i < NS; i++)  // MU0*Ms: FP64 product rounded to float32 (copypadmul2.cl:13-20)
                 bs[i] = make_float2((float)(kMu0f * (double)(a.Ms ? __fmul_rn(msm, bs[i].x) : msm)),
                                     (float)(kMu0f * (double)(a.Ms ? __fmul_rn(msm, bs[i].y) : msm)));
             if (a.vol) {
-                float2 w[NV];
+                float2 w[NS];
 #pragma unroll
-                for (int i = 0; i < NV; i++)
-                    w[i] = make_float2(__ldg(a.vol + i0 + min(xof(i), Nx - 1)), __ldg(a.vol + i0 + min(xof(i) + 1, Nx - 1)));
+                for (int i = 0; i < NS; i++) w[i] = make_float2(__ldg(a.vol + x0[i]), __ldg(a.vol + x1[i]));
 #pragma unroll
-                for (int i = 0; i < NV; i++) bs[i] = make_float2(__fmul_rn(bs[i].x, w[i].x), __fmul_rn(bs[i].y, w[i].y));
+                for (int i = 0; i < NS; i++) bs[i] = make_float2(__fmul_rn(bs[i].x, w[i].x), __fmul_rn(bs[i].y, w[i].y));
             }
 #pragma unroll
-            for (int i = 0; i < NV; i++) f[i] = make_float2(__fmul_rn(bs[i].x, f[i].x), __fmul_rn(bs[i].y, f[i].y));
+            for (int i = 0; i < NS; i++) {
+                g[i] = make_float2(__fmul_rn(bs[i].x, g[i].x), __fmul_rn(bs[i].y, g[i].y));
+                if constexpr (NPAR == 2) {
+                    const float2 o = make_float2(__shfl_xor_sync(0xffffffffu, g[i].x, 1),
+                                                 __shfl_xor_sync(0xffffffffu, g[i].y, 1));
+                    f[2 * i] = p ? o : g[i];
+                    if (2 * i + 1 < NV) f[2 * i + 1 < NV ? 2 * i + 1 : 0] = p ? g[i] : o;
+                } else {
+                    f[i] = g[i];
+                }
+            }
         }
 #pragma unroll
         for (int i = 0; i < NV; i++) {
@@ -132,6 +156,7 @@ __global__ void __launch_bounds__(4 * NPAR * Line<L>::T) k_x_fwd(const __grid_co
     cpa_wait_all();
     __syncthreads();
     line_fwd<LN, NPAR, 1, 1>(v, t, p, ex + row * S::SR + p * S::SP, 0, tw);
+    __syncthreads();  // the exchange lines become rows
 #pragma unroll
     for (int q = 0; q < LN::Qf; q++) {
         const int b = t + T * q;
@@ -165,7 +190,7 @@ __global__ void __launch_bounds__(4 * NPAR * Line<L>::T) k_x_inv(const __grid_co
     using LN = typename S::LN;
     constexpr int M = S::M, T = S::T, NT = S::NT;
     extern __shared__ __align__(16) float2 sm[];
-    float2 *tw = sm, *twr = tw + M, *ex = twr + S::WR, *Zs = ex + 4 * S::SR;
+    float2 *tw = sm, *twr = tw + M, *ex = twr + S::WR, *Zs = ex;
     const int ib = blockIdx.z;
     const int tid = threadIdx.x, p = tid % NPAR, t = (tid / NPAR) % T, row = tid / (NPAR * T);
     const int c = blockIdx.y / a.Nz, z = blockIdx.y - c * a.Nz, y0 = blockIdx.x * 4, y = y0 + row, Nx = a.Nx;
@@ -216,6 +241,7 @@ __global__ void __launch_bounds__(4 * NPAR * Line<L>::T) k_x_inv(const __grid_co
             for (int k = 0; k < LN::Rf; k++)
                 v[0][q * LN::Rf + k] = p2(Zs[row * S::ZP + NPAR * LN::freq(b, k) + p]);
     }
+    __syncthreads();  // the rows become exchange lines
     line_inv<LN, NPAR, 1, 1>(v, t, p, ex + row * S::SR + p * S::SP, 0, tw);
     float* __restrict__ B = inst_B(a, ib, c);
     const int i0 = (z * a.Ny + y) * Nx;
