@@ -363,27 +363,30 @@ __global__ void k_sum_partials(const float* __restrict__ a, const float* __restr
     }
     if (threadIdx.x == 0) part[blockIdx.x] = (double)sh_s[0] + (double)sh_c[0];
 }
-__global__ void k_sum_final(const double* part, int n, double* out) {
-    __shared__ double sh[256];
-    double s = 0.0, c = 0.0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {  // fixed order per thread (deterministic)
-        double y = part[i] - c;
-        double t = s + y;
-        c = (t - s) - y;
+// compensated FP64 sum of the partials: fixed order per thread, then a fixed tree
+// (one thread adding up the 256 threads' values was a chain of a thousand FP64
+// additions; a stage of 256x256x4 through the device ops 412 -> 410 us)
+__global__ void __launch_bounds__(256) k_sum_final(const double* part, int n, double* out) {
+    __shared__ double sh_s[256], sh_c[256];
+    auto add = [](double& s, double& c, double y, double yc) {  // s + y exactly as t + e
+        const double t = s + y, z = t - s;
+        c += yc + ((s - (t - z)) + (y - z));
         s = t;
-    }
-    sh[threadIdx.x] = s - c;
+    };
+    double s = 0.0, c = 0.0;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) add(s, c, part[i], 0.0);
+    sh_s[threadIdx.x] = s;
+    sh_c[threadIdx.x] = c;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double tot = 0.0, cc = 0.0;
-        for (int i = 0; i < blockDim.x; i++) {
-            double y = sh[i] - cc;
-            double t = tot + y;
-            cc = (t - tot) - y;
-            tot = t;
+    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
+        if (threadIdx.x < o) {
+            add(s, c, sh_s[threadIdx.x + o], sh_c[threadIdx.x + o]);
+            sh_s[threadIdx.x] = s;
+            sh_c[threadIdx.x] = c;
         }
-        *out = tot;
+        __syncthreads();
     }
+    if (threadIdx.x == 0) *out = s + c;
 }
 
 // =================================================================== host API
