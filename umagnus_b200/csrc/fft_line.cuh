@@ -16,9 +16,13 @@
 // L = R1 R2 (R3 = 1) or R1 R2 R3.  Thread t of the T threads of a line owns
 // butterflies b = t + T q of every stage.  Forward (decimation in frequency):
 //   stage 1: n = b + B1 m,            b < B1 = L/R1, m < R1  -> k1
-//   stage 2: b = k1 R3 + n3,          elements n2            -> k2
-//   stage 3: b = k1 R2 + k2,          elements n3            -> k3
-// with r = k1 + R1 k2 + R1 R2 k3.  The inverse runs the stages backwards on
+//   stage 2: b = k1 + R1 n3,          elements n2            -> k2
+//   stage 3: b = k1 + R1 k2,          elements n3            -> k3
+// with r = k1 + R1 k2 + R1 R2 k3.  k1 runs fastest, so that neighbouring
+// threads hold neighbouring frequencies (the kernel rows and half-spectrum rows
+// that they touch lie side by side in shared memory) and share the twiddles of n3
+// and k2.  With k1 slowest those were 4-way and 2-way bank conflicts in lines of
+// three stages: the field of 1024x1024 132 -> 116 us, k_y<512> of 512x512x8 130 -> 123 us (ncu).  The inverse runs the stages backwards on
 // the conjugated spectrum with the same (forward) butterflies.  A thread
 // writes, between two stages, only the slots that it read before the stage,
 // so a buffer needs one barrier per exchange.  The parity factor W_2L^(n p)
@@ -290,19 +294,18 @@ template <int L_> struct Line {
     static constexpr int Rf = three ? R3 : R2, Bf = three ? B3 : B2, Qf = three ? Q3 : Q2;
     // frequency index r of value k of final butterfly b
     __device__ __forceinline__ static int freq(int b, int k) {
-        if constexpr (three) return b / R2 + R1 * (b % R2) + R1 * R2 * k;
-        else return b + R1 * k;
+        return b + (three ? R1 * R2 : R1) * k;
     }
     static __device__ __forceinline__ int slot1(int k1, int b1) {  // b1 = n2 R3 + n3
         if constexpr (three) return k1 * P1s + (b1 / R3) * P2s + b1 % R3;
         else return k1 * P1s + b1;
     }
-    static __device__ __forceinline__ int slot2(int b2, int j) {  // b2 = k1 R3 + n3, j = n2 or k2
-        if constexpr (three) return (b2 / R3) * P1s + j * P2s + b2 % R3;
+    static __device__ __forceinline__ int slot2(int b2, int j) {  // b2 = k1 + R1 n3, j = n2 or k2
+        if constexpr (three) return (b2 % R1) * P1s + j * P2s + b2 / R1;
         else return b2 * P1s + j;
     }
-    static __device__ __forceinline__ int slot3(int b3, int j) {  // b3 = k1 R2 + k2, j = n3
-        return (b3 / R2) * P1s + (b3 % R2) * P2s + j;
+    static __device__ __forceinline__ int slot3(int b3, int j) {  // b3 = k1 + R1 k2, j = n3
+        return (b3 % R1) * P1s + (b3 / R1) * P2s + j;
     }
 };
 
@@ -409,7 +412,7 @@ __device__ __forceinline__ void line_fwd(P2 (&v)[NC][LN::NE], int t, int p, floa
 #pragma unroll
                 for (int k2 = 1; k2 < R2; k2++) {
                     P2 rr, ii;
-                    tw_pair(tw[NPAR * R1 * k2 * (b % R3)], rr, ii);
+                    tw_pair(tw[NPAR * R1 * k2 * (b / R1)], rr, ii);
 #pragma unroll
                     for (int c = 0; c < NC; c++) v[c][q * R2 + k2] = pcmul(v[c][q * R2 + k2], rr, ii);
                 }
@@ -457,7 +460,7 @@ __device__ __forceinline__ void line_inv(P2 (&v)[NC][LN::NE], int t, int p, floa
 #pragma unroll
                 for (int j = 1; j < R3; j++) {
                     P2 rr, ii;
-                    tw_pair(tw[NPAR * R1 * (b % R2) * j], rr, ii);
+                    tw_pair(tw[NPAR * R1 * (b / R1) * j], rr, ii);
 #pragma unroll
                     for (int c = 0; c < NC; c++) v[c][q * R3 + j] = pcmul(v[c][q * R3 + j], rr, ii);
                 }
@@ -488,9 +491,9 @@ __device__ __forceinline__ void line_inv(P2 (&v)[NC][LN::NE], int t, int p, floa
     line_butterflies<LN, R2, LN::Q2, NC>(v);  // over k2 -> n2
 #pragma unroll
     for (int q = 0; q < LN::Q2; q++) {
-        const int b = t + T * q;  // k1 R3 + n3
+        const int b = t + T * q;  // k1 + R1 n3
         if (LN::B2 % T == 0 || b < LN::B2) {
-            const int kp = NPAR * (b / R3) + p, n3 = b % R3;
+            const int kp = NPAR * (b % R1) + p, n3 = b / R1;
 #pragma unroll
             for (int j = 0; j < R2; j++) {
                 if (!LN::three && j == 0) continue;  // n = 0
