@@ -42,13 +42,11 @@ CONFIG = dict(N=(256, 256, 16), cell=(2e-9, 2e-9, 1e-9), Ms=1.1e6, Aex=1.6e-11, 
               anisU=(0.0, 0.0, 1.0), alpha=0.3, B_ext=(0.0, 0.0, 0.05), seed=2)
 METRIC = "RK45DP cell-updates/s (256x256x16 multilayer, FP32, Newell demag)"
 UNIT = "cell-updates/s"
-# dram__bytes_read.sum + dram__bytes_write.sum of one k_reg_b<512,4> launch on
-# this workload (79,939,328 + 4,860,160 B), from one ncu --set full capture of
-# that launch with packed FP32 butterflies and staged twiddle tables (cold
-# cache: ncu flushes the caches between its passes)
-TRAFFIC_B = 84799488
-TRAFFIC_B_SOURCE = ("ncu capture of k_reg_b<512,4>, packed FP32 butterflies + staged twiddle tables "
-                    "(profiles/k_reg_b_multilayer_256x256x16.md)")
+# dram__bytes.sum.per_second x gpu__time_duration.sum of one k_y<256,2> launch on
+# this mesh (1.693274 TB/s x 50.624 us), from one ncu capture (cold cache: ncu
+# flushes the caches between its passes)
+TRAFFIC_B = 85720303
+TRAFFIC_B_SOURCE = "ncu capture of k_y<256,2> (profiles/k_y_512x512x8_and_256x256x16.md)"
 
 
 def alg_bytes_per_eval(N):
@@ -404,7 +402,7 @@ def run_ours(args, rank, world, local_rank):
                        "l2": "working set ~0.2 GB > 126 MB L2, no flush", "parallelism": f"replicas x{world}",
                        "graph_steps": graph_steps, "warmup_steps_done": warm, "launch_shapes": tuning,
                        "autotuned": not args.no_autotune},
-            "roofline": {"bound": "hbm", "kernel": f"k_reg_b (demag pass B: y FFT, kernel multiply, inverse y)",
+            "roofline": {"bound": "hbm", "kernel": "k_y (demag pass B: y FFT, kernel multiply, inverse y)",
                          "achieved": bp["B"] / (ms_pass["B"] * 1e-3) / 1e9, "peak": peak, "peak_source": peak_kind,
                          "unit": "GB/s", "frac": bp["B"] / (ms_pass["B"] * 1e-3) / 1e9 / peak,
                          "traffic": TRAFFIC_B, "traffic_source": TRAFFIC_B_SOURCE,
