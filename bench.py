@@ -224,13 +224,20 @@ def time_ref(r, max_steps, budget_s):
     return time.perf_counter() - t0, n, r.nsteps - acc0
 
 
+def ref_unavailable():
+    """Why the reference's kernels cannot be run, or None."""
+    from oracle import clref
+    if clref.available():
+        return None
+    return "the reference's kernels are not built for the host (their source tree was absent at build time)"
+
+
 def cpu_baseline(config, budget_s=12.0):
     """Bounded sample of the workload on the host cores: the reference's own
     kernels (oracle/_ref, host threads) + scipy FFT, one warm-up step, then
     whole RK45DP steps for about budget_s seconds."""
-    from oracle import clref
-    if not clref.available():
-        raise RuntimeError("oracle/_ref/libclref.so is not built (run __graft_entry__.build())")
+    if ref_unavailable():
+        return {"unavailable": ref_unavailable()}
     r = make_ref(config)
     r.step()
     t, n, acc = time_ref(r, 10 ** 6, budget_s)
@@ -1124,6 +1131,9 @@ def main():
     local_rank = int(os.environ.get("LOCAL_RANK", "0"))
     if args.impl == "reference":
         if rank != 0:
+            return 0
+        if ref_unavailable():
+            print(json.dumps({"impl": "reference", "unavailable": ref_unavailable()}), flush=True)
             return 0
         r = make_ref(CONFIG)
         for _ in range(min(max(args.warmup, 1), 2)):  # bounded warm-up: a CPU step takes seconds
