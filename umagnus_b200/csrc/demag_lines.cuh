@@ -370,7 +370,8 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
 // the forward transform runs.  Four columns a CTA: 32-byte pieces times Ny rows
 // are one contiguous run.  256x256x16 is bound by issue and shared memory at 12
 // warps per SM: 45 us where a 512-point transform in three radix-8 stages took
-// 50.5; 512x512x32 by its 1.0 GB (480 us; 1538 us with two columns a CTA,
+// 50.5; 512x512x32 by the two exchanges of
+// its longer lines (L1 at 67 %, DRAM at a quarter; 1538 us with two columns a CTA,
 // whose 16-byte pieces move twice the sectors); small films by one CTA's
 // latency (128x128: 4.6 us against 8.3; 250x250: 6.7 against 38.9).
 // Kernel components in shared memory: xx yy zz xy (one layer), then yz xz.

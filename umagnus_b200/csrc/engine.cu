@@ -981,7 +981,8 @@ static thread_local cudaStream_t g_launch_stream = nullptr;
 static cudaStream_t S() { return g_launch_stream ? g_launch_stream : ctx().stream; }
 // Kernels of one simulation overlap the next one's start (common.cuh); those
 // of an ensemble do not: waiting CTAs would hold the room that the other
-// classes' kernels, on streams of their own, can use.
+// classes' kernels, on streams of their own, can use (48 films: 23.1 ms, 29.0 with
+// it).  A general instance's demag passes still overlap among themselves.
 static bool overlap(const SimImpl* s) { return !s->batched && !g_launch_stream; }
 static unsigned ctl_grid(const SimImpl* s) { return (unsigned)((s->nb + 127) / 128); }
 
